@@ -28,6 +28,7 @@
 
 #include "internal.h"
 #include "box.cuh"
+#include "clip.cuh"
 #include "ptx.cuh"
 
 namespace mdsm {
@@ -832,40 +833,6 @@ __device__ __forceinline__ void cta_done(unsigned *done, int b, int phase)
     if (threadIdx.x == 0) atomicAdd(&done[3 * b + phase], 1u);
 }
 
-// The clip test of the standalone clip (rfi.cu), fabs(v - mean) >= lim in double, is monotone
-// in v on each side of the mean (the rounded difference is monotone), so for integer samples
-// it holds exactly for v >= hi when v >= ceil(mean) and for v <= lo below: the bounds are found
-// from the real-valued estimates and corrected with that same test.
-__device__ __forceinline__ void clip_bounds_u8(double mu, double lim, int *cm, int *lo, int *hi)
-{
-    auto clipped = [&](int v) { return fabs(__dadd_rn((double)v, -mu)) >= lim; };
-    const int c = (int)ceil(mu);
-    int h = (int)fmin(fmax(ceil(mu + lim), (double)c), 256.0);
-    while (h > c && clipped(h - 1)) --h;
-    while (h <= 255 && !clipped(h)) ++h;
-    int l = (int)fmax(fmin(floor(mu - lim), (double)(c - 1)), -1.0);
-    while (l < c - 1 && clipped(l + 1)) ++l;
-    while (l >= 0 && !clipped(l)) --l;
-    *cm = c;
-    *lo = l;
-    *hi = h;
-}
-
-__device__ __forceinline__ uint8_t clip_rep_u8(double mu)
-{
-    const int r = __double2int_rn(mu);
-    return (uint8_t)min(max(r, 0), 255);
-}
-
-__device__ __forceinline__ void mean_sigma_ll(long long s1, long long s2, long long n, double *mu,
-                                              double *sig)
-{
-    const double m = __ddiv_rn((double)s1, (double)n);
-    const double var = __dadd_rn(__ddiv_rn((double)s2, (double)n), -__dmul_rn(m, m));
-    *mu = m;
-    *sig = var > 0.0 ? __dsqrt_rn(var) : 0.0;
-}
-
 // Phase 3's item source: the dedispersion list, each item waiting for its beam's clip (when
 // there is one), each compute warp counting its stores (when a search follows).
 struct FusedItems {
@@ -947,12 +914,12 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
                 mean_sigma_ll(s1, s2, B.ncols, &s_mu, &s_sig);
             }
             __syncthreads();
-            int cm, lo, hi;
-            clip_bounds_u8(s_mu, __dmul_rn(f.k_chan, s_sig), &cm, &lo, &hi);
-            const uint8_t rep = clip_rep_u8(s_mu);
+            int lo, hi;
+            clip_bounds_int<0, 255>(s_mu, __dmul_rn(f.k_chan, s_sig), &lo, &hi);
+            const uint8_t rep = (uint8_t)clip_rep_int<0, 255>(s_mu);
             for (long long i = tid; i < B.ncols; i += Cfg::THREADS) {
                 const int v = row[i];
-                if (v >= cm ? v >= hi : v <= lo) row[i] = rep;
+                if (v <= lo || v >= hi) row[i] = rep;
             }
             cta_done(f.done, w.x, 0);
         }
@@ -975,14 +942,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
             }
             double mu, sig;
             mean_sigma_ll(s1, s2, B.nchans, &mu, &sig);
-            int cm, lo, hi;
-            clip_bounds_u8(mu, __dmul_rn(f.k_spec, sig), &cm, &lo, &hi);
-            const uint8_t rep = clip_rep_u8(mu);
+            int lo, hi;
+            clip_bounds_int<0, 255>(mu, __dmul_rn(f.k_spec, sig), &lo, &hi);
+            const uint8_t rep = (uint8_t)clip_rep_int<0, 255>(mu);
             uint8_t *cw = B.in + t;
             for (int c = 0; c < B.nchans; ++c) {
                 uint8_t *p = cw + (size_t)c * (size_t)B.in_stride;
                 const int v = *p;
-                if (v >= cm ? v >= hi : v <= lo) *p = rep;
+                if (v <= lo || v >= hi) *p = rep;
             }
         }
         cta_done(f.done, w.x, 1);

@@ -7,197 +7,714 @@
 // |x - mean| <= sigma/4 (:61).  Statistics are exact for integer samples (int64 sums) and use
 // a fixed left-to-right order of double sums for float samples, so the device result equals
 // the oracle's bit for bit.
+//
+// The double operations of the clip test are the slow pipe of this GPU (2 lanes per clock per
+// SM), so a row's test is turned once into two bounds of the sample type (clip.cuh) and the
+// samples are compared as integers or floats; the float statistics keep the two double
+// operations a sample that their rounding needs.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <type_traits>
+
+#include "clip.cuh"
 #include "internal.h"
 
 namespace mdsm {
 
-template <typename T>
-struct Clip;
+namespace cg = cooperative_groups;
 
+namespace {
+
+template <typename T>
+struct Range;
 template <>
-struct Clip<uint8_t> {
-    static __device__ __forceinline__ uint8_t from(double v)
-    {
-        int r = __double2int_rn(v);
-        return (uint8_t)min(max(r, 0), 255);
-    }
+struct Range<uint8_t> {
+    static constexpr int lo = 0, hi = 255;
 };
 template <>
-struct Clip<uint16_t> {
-    static __device__ __forceinline__ uint16_t from(double v)
-    {
-        int r = __double2int_rn(v);
-        return (uint16_t)min(max(r, 0), 65535);
-    }
+struct Range<uint16_t> {
+    static constexpr int lo = 0, hi = 65535;
 };
 template <>
-struct Clip<int16_t> {
-    static __device__ __forceinline__ int16_t from(double v)
-    {
-        int r = __double2int_rn(v);
-        return (int16_t)min(max(r, -32768), 32767);
-    }
+struct Range<int16_t> {
+    static constexpr int lo = -32768, hi = 32767;
 };
-template <>
-struct Clip<float> {
-    static __device__ __forceinline__ float from(double v) { return __double2float_rn(v); }
+
+struct IntClip {
+    int lo, hi, rep;  // v <= lo or v >= hi is replaced by rep
 };
 
 template <typename T>
-constexpr bool is_int_sample()
+__device__ __forceinline__ IntClip int_clip(long long s1, long long s2, long long n, double k)
 {
-    return !std::is_same<T, float>::value;
+    double mu, sig;
+    mean_sigma_ll(s1, s2, n, &mu, &sig);
+    IntClip c;
+    clip_bounds_int<Range<T>::lo, Range<T>::hi>(mu, __dmul_rn(k, sig), &c.lo, &c.hi);
+    c.rep = clip_rep_int<Range<T>::lo, Range<T>::hi>(mu);
+    return c;
 }
 
-__device__ __forceinline__ void mean_sigma_int(long long s1, long long s2, long long n, double *mu,
-                                               double *sig)
+// The samples of one 32-bit word: SPW samples, sample e in bits [e * 8 * size, ...).
+template <typename T>
+__device__ __forceinline__ int word_sample(uint32_t w, int e)
 {
-    const double m = __ddiv_rn((double)s1, (double)n);
-    const double var = __dadd_rn(__ddiv_rn((double)s2, (double)n), -__dmul_rn(m, m));
-    *mu = m;
-    *sig = var > 0.0 ? __dsqrt_rn(var) : 0.0;
+    if constexpr (sizeof(T) == 1)
+        return (int)((w >> (8 * e)) & 0xffu);
+    else if constexpr (std::is_same<T, int16_t>::value)
+        return (int)(int16_t)(w >> (16 * e));
+    else
+        return (int)((w >> (16 * e)) & 0xffffu);
 }
 
-// One CTA per channel: statistics over the row, then the clip.
+// Bounds of a word's samples, ready to test the word (each sample its own bounds).
+// uint8: the even and odd bytes as 16-bit lanes; a lane x plus 256 - b has bit 8 set when
+// x >= b, so one 32-bit add tests two samples against a bound each.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    k_clip_channels(T *__restrict__ x, long long stride, long long len, double k)
+struct WordClip {
+    IntClip c[2];
+    __device__ __forceinline__ void set(const IntClip *s)
+    {
+        c[0] = s[0];
+        c[1] = s[1];
+    }
+    // w with its clipped samples replaced
+    __device__ __forceinline__ uint32_t apply(uint32_t w) const
+    {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int v = word_sample<T>(w, e);
+            if (v <= c[e].lo || v >= c[e].hi)
+                w = (w & ~(0xffffu << (16 * e))) | ((uint32_t)(uint16_t)c[e].rep << (16 * e));
+        }
+        return w;
+    }
+};
+template <>
+struct WordClip<uint8_t> {
+    uint32_t in_e, out_e, in_o, out_o, rep;
+    __device__ __forceinline__ void set(const IntClip *s)
+    {
+        auto lanes = [](int a, int b) { return (uint32_t)(256 - a) | ((uint32_t)(256 - b) << 16); };
+        in_e = lanes(s[0].lo + 1, s[2].lo + 1);
+        out_e = lanes(s[0].hi, s[2].hi);
+        in_o = lanes(s[1].lo + 1, s[3].lo + 1);
+        out_o = lanes(s[1].hi, s[3].hi);
+        rep = (uint32_t)s[0].rep | ((uint32_t)s[1].rep << 8) | ((uint32_t)s[2].rep << 16) |
+              ((uint32_t)s[3].rep << 24);
+    }
+    __device__ __forceinline__ uint32_t apply(uint32_t w) const
+    {
+        const uint32_t e = w & 0x00ff00ffu, o = __byte_perm(w, 0u, 0x4341);
+        const uint32_t be = ((e + out_e) | ~(e + in_e)) & 0x01000100u;
+        const uint32_t bo = ((o + out_o) | ~(o + in_o)) & 0x01000100u;
+        if ((be | bo) == 0u) return w;
+        const uint32_t m = (be >> 8) * 0xffu | bo * 0xffu;
+        return (w & ~m) | (rep & m);
+    }
+};
+
+// Sums of a word's samples and of their squares (32-bit s1; s2 as wide as the caller's).
+template <typename T>
+__device__ __forceinline__ void word_sums(uint32_t w, int &s1, unsigned long long &s2)
 {
-    extern __shared__ __align__(16) unsigned char sm[];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int v = word_sample<T>(w, e);
+        s1 += v;
+        s2 += (unsigned long long)((uint32_t)v * (uint32_t)v);  // (|v| < 2^16: 32 bits hold it)
+    }
+}
+
+constexpr int kChanThreads = 512;
+
+// One CTA per channel: exact statistics over the row, then the clip.  The row is read twice in
+// 16-byte vectors (dp4a sums for uint8); the second read comes from L2 (the rows in flight are
+// far below its size), so the DRAM traffic is one read plus the vectors that change.  On uint8
+// 4096 ch x 97921 this replaced one byte a thread and three double operations a sample.
+template <typename T>
+__global__ void __launch_bounds__(kChanThreads)
+    k_clip_channels_int(T *__restrict__ x, long long stride, long long len, double k)
+{
+    constexpr int N = 16 / (int)sizeof(T);
     T *row = x + (size_t)blockIdx.x * stride;
-    __shared__ double s_mu, s_sig;
-    if constexpr (is_int_sample<T>()) {
-        __shared__ long long r1[256], r2[256];
-        long long a1 = 0, a2 = 0;
-        for (long long i = threadIdx.x; i < len; i += blockDim.x) {
-            const long long v = (long long)row[i];
-            a1 += v;
-            a2 += v * v;
-        }
-        r1[threadIdx.x] = a1;
-        r2[threadIdx.x] = a2;
-        __syncthreads();
-        for (int o = 128; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) {
-                r1[threadIdx.x] += r1[threadIdx.x + o];
-                r2[threadIdx.x] += r2[threadIdx.x + o];
+    const int tid = threadIdx.x;
+    // samples before the first 16-byte boundary, whole vectors, the rest
+    const long long head =
+        min(len, (long long)(((16 - ((uintptr_t)row & 15)) & 15) / sizeof(T)));
+    uint4 *vec = reinterpret_cast<uint4 *>(row + head);
+    const long long nv = (len - head) / N, tail = head + nv * N;
+    long long a1 = 0;
+    unsigned long long a2 = 0;
+    auto one = [&](long long i) {
+        const long long v = row[i];
+        a1 += v;
+        a2 += (unsigned long long)(v * v);
+    };
+    for (long long i = tid; i < head; i += kChanThreads) one(i);
+    for (long long i = tail + tid; i < len; i += kChanThreads) one(i);
+    if constexpr (sizeof(T) == 1) {
+        // 32-bit sums of at most 1024 vectors (16384 * 255^2 < 2^32)
+        for (long long i0 = tid; i0 < nv; i0 += 1024LL * kChanThreads) {
+            uint32_t s1 = 0, s2 = 0;
+            const long long i1 = min(nv, i0 + 1024LL * kChanThreads);
+#pragma unroll 4
+            for (long long i = i0; i < i1; i += kChanThreads) {
+                const uint4 v = vec[i];
+                s1 = __dp4a(v.x, 0x01010101u, s1);
+                s1 = __dp4a(v.y, 0x01010101u, s1);
+                s1 = __dp4a(v.z, 0x01010101u, s1);
+                s1 = __dp4a(v.w, 0x01010101u, s1);
+                s2 = __dp4a(v.x, v.x, s2);
+                s2 = __dp4a(v.y, v.y, s2);
+                s2 = __dp4a(v.z, v.z, s2);
+                s2 = __dp4a(v.w, v.w, s2);
             }
-            __syncthreads();
+            a1 += s1;
+            a2 += s2;
         }
-        if (threadIdx.x == 0) mean_sigma_int(r1[0], r2[0], len, &s_mu, &s_sig);
     } else {
-        // runs of 1024 summed left to right, partials summed left to right
-        double2 *part = reinterpret_cast<double2 *>(sm);
-        const long long nch = (len + 1023) / 1024;
-        for (long long c = threadIdx.x; c < nch; c += blockDim.x) {
-            const long long c0 = c * 1024, c1 = min(c0 + 1024, len);
-            double p1 = 0.0, p2 = 0.0;
-            for (long long i = c0; i < c1; ++i) {
-                const double v = (double)row[i];
-                p1 = __dadd_rn(p1, v);
-                p2 = __fma_rn(v, v, p2);  // v*v exact: same as dmul + dadd
+        for (long long i0 = tid; i0 < nv; i0 += 1024LL * kChanThreads) {
+            int s1 = 0;  // (8192 samples of at most 65535)
+            const long long i1 = min(nv, i0 + 1024LL * kChanThreads);
+#pragma unroll 4
+            for (long long i = i0; i < i1; i += kChanThreads) {
+                const uint4 v = vec[i];
+                word_sums<T>(v.x, s1, a2);
+                word_sums<T>(v.y, s1, a2);
+                word_sums<T>(v.z, s1, a2);
+                word_sums<T>(v.w, s1, a2);
             }
-            part[c] = make_double2(p1, p2);
+            a1 += s1;
         }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s1 = 0.0, s2 = 0.0;
-            for (long long c = 0; c < nch; ++c) {
-                s1 = __dadd_rn(s1, part[c].x);
-                s2 = __dadd_rn(s2, part[c].y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+    __shared__ long long r1[kChanThreads / 32];
+    __shared__ unsigned long long r2[kChanThreads / 32];
+    __shared__ IntClip s_c;
+    if ((tid & 31) == 0) {
+        r1[tid >> 5] = a1;
+        r2[tid >> 5] = a2;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kChanThreads / 32; ++w) {
+            a1 += r1[w];
+            a2 += r2[w];
+        }
+        s_c = int_clip<T>(a1, (long long)a2, len, k);
+    }
+    __syncthreads();
+    const IntClip c = s_c;
+    auto clip_one = [&](long long i) {
+        const int v = row[i];
+        if (v <= c.lo || v >= c.hi) row[i] = (T)c.rep;
+    };
+    for (long long i = tid; i < head; i += kChanThreads) clip_one(i);
+    for (long long i = tail + tid; i < len; i += kChanThreads) clip_one(i);
+    WordClip<T> wc;
+    const IntClip c4[4] = {c, c, c, c};
+    wc.set(c4);
+#pragma unroll 4
+    for (long long i = tid; i < nv; i += kChanThreads) {
+        const uint4 v = vec[i];
+        const uint4 q = make_uint4(wc.apply(v.x), wc.apply(v.y), wc.apply(v.z), wc.apply(v.w));
+        if (((q.x ^ v.x) | (q.y ^ v.y) | (q.z ^ v.z) | (q.w ^ v.w)) != 0u) vec[i] = q;
+    }
+}
+
+constexpr int kSpecThreads = 512;  // 256 channels x 2 vectors of 16 bytes
+
+// Spectra of integer samples: a cluster of CTAs takes 32 bytes of columns (32 uint8 spectra, 16
+// of 16-bit samples) over all channels.  A thread holds the same 16-byte vector of NV channels
+// in registers from the statistics to the clip, so the block is read once and only the vectors
+// that change are written; the CTAs of the cluster (each 256 NV channels) add their columns'
+// sums over distributed shared memory.  Past 8 x 2048 channels the threads take further batches
+// of channels and read them again for the clip.  Rows start on 16-byte boundaries; columns at
+// or past len are neither counted nor written.
+template <typename T, int NV>
+__global__ void __launch_bounds__(kSpecThreads, 2)
+    k_clip_spectra_int(T *__restrict__ x, int nchans, long long stride, long long len, double k,
+                       int nbatch)
+{
+    constexpr int SPW = 4 / (int)sizeof(T);  // samples per word
+    constexpr int N = 4 * SPW;               // columns of a vector
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), nrank = (int)cl.num_blocks();
+    const int tid = threadIdx.x, half = tid & 1;
+    const long long t0 = (long long)(blockIdx.x / nrank) * (2 * N) + half * N;
+    const int ncol = (int)max(0LL, min((long long)N, len - t0));  // columns of this vector
+    __shared__ unsigned long long sum1[2 * N], sum2[2 * N];
+    __shared__ IntClip clip[2 * N];
+    if (tid < 2 * N) sum1[tid] = sum2[tid] = 0ull;
+    __syncthreads();
+
+    uint32_t v[NV][4];
+    auto channel = [&](int b, int i) {
+        return ((b * nrank + rank) * NV + i) * (kSpecThreads / 2) + (tid >> 1);
+    };
+    auto load = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = channel(b, i);
+            uint4 q = make_uint4(0u, 0u, 0u, 0u);  // (adds nothing)
+            if (c < nchans) {
+                const T *p = x + (size_t)c * (size_t)stride + t0;
+                if (ncol == N) {
+                    q = *reinterpret_cast<const uint4 *>(p);
+                } else {
+                    uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                    for (int e = 0; e < N; ++e)
+                        if (e < ncol)
+                            w[e / SPW] |= ((uint32_t)p[e] & (0xffffffffu >> (32 - 8 * sizeof(T))))
+                                          << (8 * sizeof(T) * (e % SPW));
+                    q = make_uint4(w[0], w[1], w[2], w[3]);
+                }
             }
-            const double m = __ddiv_rn(s1, (double)len);
-            const double var = __dadd_rn(__ddiv_rn(s2, (double)len), -__dmul_rn(m, m));
-            s_mu = m;
-            s_sig = var > 0.0 ? __dsqrt_rn(var) : 0.0;
+            v[i][0] = q.x;
+            v[i][1] = q.y;
+            v[i][2] = q.z;
+            v[i][3] = q.w;
+        }
+    };
+    for (int b = 0; b < nbatch; ++b) {
+        load(b);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            // the word's columns summed over this thread's channels, then over the 16 lanes of
+            // the warp that hold the same columns
+            if constexpr (sizeof(T) == 1) {
+                uint32_t p01 = 0, p23 = 0, s2[4] = {0u, 0u, 0u, 0u};
+                constexpr int G = (NV + 3) / 4;
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    // four channels' words as one word per column: dp4a adds the four samples
+                    // (and their squares)
+                    const uint32_t a = v[4 * g][w];
+                    const uint32_t bb = 4 * g + 1 < NV ? v[(4 * g + 1) % NV][w] : 0u;
+                    const uint32_t c = 4 * g + 2 < NV ? v[(4 * g + 2) % NV][w] : 0u;
+                    const uint32_t d = 4 * g + 3 < NV ? v[(4 * g + 3) % NV][w] : 0u;
+                    const uint32_t ab0 = __byte_perm(a, bb, 0x5140), ab2 = __byte_perm(a, bb, 0x7362);
+                    const uint32_t cd0 = __byte_perm(c, d, 0x5140), cd2 = __byte_perm(c, d, 0x7362);
+                    const uint32_t col[4] = {
+                        __byte_perm(ab0, cd0, 0x5410), __byte_perm(ab0, cd0, 0x7632),
+                        __byte_perm(ab2, cd2, 0x5410), __byte_perm(ab2, cd2, 0x7632)};
+                    p01 = __dp4a(col[0], 0x01010101u, p01);
+                    p01 += __dp4a(col[1], 0x01010101u, 0u) << 16;
+                    p23 = __dp4a(col[2], 0x01010101u, p23);
+                    p23 += __dp4a(col[3], 0x01010101u, 0u) << 16;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s2[e] = __dp4a(col[e], col[e], s2[e]);
+                }
+                // (16-bit lanes: 16 lanes x NV channels x 255 < 2^16)
+                static_assert(16 * NV * 255 < 65536, "packed column sums");
+#pragma unroll
+                for (int o = 16; o > 1; o >>= 1) {
+                    p01 += __shfl_xor_sync(0xffffffffu, p01, o);
+                    p23 += __shfl_xor_sync(0xffffffffu, p23, o);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s2[e] += __shfl_xor_sync(0xffffffffu, s2[e], o);
+                }
+                if ((tid & 31) < 2) {
+                    const int q = half * N + 4 * w;
+                    atomicAdd(&sum1[q], (unsigned long long)(p01 & 0xffffu));
+                    atomicAdd(&sum1[q + 1], (unsigned long long)(p01 >> 16));
+                    atomicAdd(&sum1[q + 2], (unsigned long long)(p23 & 0xffffu));
+                    atomicAdd(&sum1[q + 3], (unsigned long long)(p23 >> 16));
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) atomicAdd(&sum2[q + e], (unsigned long long)s2[e]);
+                }
+            } else {
+                int s1[2] = {0, 0};
+                unsigned long long s2[2] = {0ull, 0ull};
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int u = word_sample<T>(v[i][w], e);
+                        s1[e] += u;
+                        s2[e] += (unsigned long long)((uint32_t)u * (uint32_t)u);
+                    }
+#pragma unroll
+                for (int o = 16; o > 1; o >>= 1)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        s1[e] += __shfl_xor_sync(0xffffffffu, s1[e], o);
+                        s2[e] += __shfl_xor_sync(0xffffffffu, s2[e], o);
+                    }
+                if ((tid & 31) < 2)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        atomicAdd(&sum1[half * N + 2 * w + e], (unsigned long long)(long long)s1[e]);
+                        atomicAdd(&sum2[half * N + 2 * w + e], s2[e]);
+                    }
+            }
         }
     }
     __syncthreads();
-    const double mu = s_mu, lim = __dmul_rn(k, s_sig);
-    const T rep = Clip<T>::from(mu);
-    for (long long i = threadIdx.x; i < len; i += blockDim.x) {
-        const double v = (double)row[i];
-        if (fabs(__dadd_rn(v, -mu)) >= lim) row[i] = rep;
+    cl.sync();  // every CTA's sums are complete
+    if (tid < 2 * N) {
+        unsigned long long s1 = 0, s2 = 0;
+        for (int r = 0; r < nrank; ++r) {
+            s1 += *cl.map_shared_rank(&sum1[tid], r);
+            s2 += *cl.map_shared_rank(&sum2[tid], r);
+        }
+        clip[tid] = int_clip<T>((long long)s1, (long long)s2, nchans, k);
+    }
+    cl.sync();  // no CTA leaves while another reads its sums; clip[] is visible to its own CTA
+    for (int b = 0; b < nbatch; ++b) {
+        if (nbatch > 1) load(b);
+        uint32_t changed = 0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            WordClip<T> wc;
+            wc.set(&clip[half * N + SPW * w]);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                const uint32_t q = wc.apply(v[i][w]);
+                changed |= (uint32_t)(q != v[i][w]) << i;
+                v[i][w] = q;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int c = channel(b, i);
+            if (!((changed >> i) & 1u) || c >= nchans) continue;
+            T *p = x + (size_t)c * (size_t)stride + t0;
+            if (ncol == N) {
+                *reinterpret_cast<uint4 *>(p) = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < N; ++e)
+                    if (e < ncol) p[e] = (T)word_sample<T>(v[i][e / SPW], e % SPW);
+            }
+        }
     }
 }
 
-// One thread per time sample: statistics over the channels, then the clip.
+// Spectra of integer samples whose rows do not start on 16-byte boundaries: one thread per time
+// sample.
 template <typename T>
-__global__ void k_clip_spectra(T *__restrict__ x, int nchans, long long stride, long long len,
-                               double k)
+__global__ void k_clip_spectra_any(T *__restrict__ x, int nchans, long long stride, long long len,
+                                   double k)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= len) return;
-    double mu, sig;
-    if constexpr (is_int_sample<T>()) {
-        long long s1 = 0, s2 = 0;
-        for (int c = 0; c < nchans; ++c) {
-            const long long v = (long long)x[(size_t)c * stride + t];
-            s1 += v;
-            s2 += v * v;
-        }
-        mean_sigma_int(s1, s2, nchans, &mu, &sig);
-    } else {
-        double s1 = 0.0, s2 = 0.0;
-        for (int c0 = 0; c0 < nchans; c0 += 1024) {
-            const int c1 = min(c0 + 1024, nchans);
-            double p1 = 0.0, p2 = 0.0;
-            for (int c = c0; c < c1; ++c) {
-                const double v = (double)x[(size_t)c * stride + t];
-                p1 = __dadd_rn(p1, v);
-                p2 = __fma_rn(v, v, p2);  // v*v exact: same as dmul + dadd
-            }
-            s1 = __dadd_rn(s1, p1);
-            s2 = __dadd_rn(s2, p2);
-        }
-        mu = __ddiv_rn(s1, (double)nchans);
-        const double var = __dadd_rn(__ddiv_rn(s2, (double)nchans), -__dmul_rn(mu, mu));
-        sig = var > 0.0 ? __dsqrt_rn(var) : 0.0;
+    long long s1 = 0, s2 = 0;
+    for (int c = 0; c < nchans; ++c) {
+        const long long v = (long long)x[(size_t)c * stride + t];
+        s1 += v;
+        s2 += v * v;
     }
-    const double lim = __dmul_rn(k, sig);
-    const T rep = Clip<T>::from(mu);
+    const IntClip cb = int_clip<T>(s1, s2, nchans, k);
     for (int c = 0; c < nchans; ++c) {
         T *p = x + (size_t)c * stride + t;
-        if (fabs(__dadd_rn((double)*p, -mu)) >= lim) *p = rep;
+        const int v = *p;
+        if (v <= cb.lo || v >= cb.hi) *p = (T)cb.rep;
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// float samples
+// ------------------------------------------------------------------------------------------
+constexpr int kRun = 1024;  // samples of a left-to-right run
+
+// A normal float as a double by integer operations (the conversion instruction runs at the
+// double rate); `special` when the exponent field is 0 or 255.
+__device__ __forceinline__ double float_bits_double(uint32_t b)
+{
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)),
+                            (int)(b << 29));
+}
+__device__ __forceinline__ uint32_t special_key(float x)
+{
+    return (__float_as_uint(x) & 0x7f800000u) - 0x00800000u;  // >= 0x7f000000: special
+}
+
+// p1 += v, p2 += v * v (v * v is exact in double: one rounding each, as dmul + dadd) over U
+// consecutive samples.
+template <int U>
+__device__ __forceinline__ void run_add(const float (&v)[U], double &p1, double &p2)
+{
+    uint32_t sp = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j) sp = max(sp, special_key(v[j]));
+    if (sp < 0x7f000000u) {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const double d = float_bits_double(__float_as_uint(v[j]));
+            p1 = __dadd_rn(p1, d);
+            p2 = __fma_rn(d, d, p2);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const double d = (double)v[j];
+            p1 = __dadd_rn(p1, d);
+            p2 = __fma_rn(d, d, p2);
+        }
+    }
+}
+
+struct FloatClip {
+    float lo, hi, rep;
+};
+
+__device__ __forceinline__ FloatClip float_clip(double s1, double s2, double n, double k)
+{
+    const double mu = __ddiv_rn(s1, n);
+    const double var = __dadd_rn(__ddiv_rn(s2, n), -__dmul_rn(mu, mu));
+    const double sig = var > 0.0 ? __dsqrt_rn(var) : 0.0;
+    FloatClip c;
+    clip_bounds_f32(mu, __dmul_rn(k, sig), &c.lo, &c.hi);
+    c.rep = __double2float_rn(mu);
+    return c;
+}
+
+constexpr int kChanF32Threads = 128;
+
+// Channels of float samples: a CTA takes `rpc` rows, one thread per run of 1024 samples of a
+// row (left to right), then the runs' sums left to right, then the clip in float.  Several rows
+// a CTA because a warp of double operations costs the same with few lanes as with 32.
+__global__ void __launch_bounds__(kChanF32Threads)
+    k_clip_channels_f32(float *__restrict__ x, int nchans, long long stride, long long len,
+                        double k, int rpc)
+{
+    extern __shared__ __align__(16) unsigned char sm[];
+    double2 *part = reinterpret_cast<double2 *>(sm);  // [rpc][nruns]
+    __shared__ FloatClip clip[kChanF32Threads];
+    const int tid = threadIdx.x;
+    const int c0 = blockIdx.x * rpc, rows = min(rpc, nchans - c0);
+    const int nruns = (int)((len + kRun - 1) / kRun);
+    const bool vec = (((uintptr_t)x | (uintptr_t)(stride * 4)) & 15) == 0;
+    for (int q = tid; q < rows * nruns; q += kChanF32Threads) {
+        const int r = q / nruns;
+        const long long i0 = (long long)(q - r * nruns) * kRun;
+        const float *p = x + (size_t)(c0 + r) * (size_t)stride + i0;
+        const int n = (int)min((long long)kRun, len - i0);
+        double p1 = 0.0, p2 = 0.0;
+        int i = 0;
+        if (vec) {
+            float4 q0[4], q1[4];
+            auto ld = [&](float4 (&d)[4], int at) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d[j] = *reinterpret_cast<const float4 *>(p + at + 4 * j);
+            };
+            auto add = [&](const float4 (&d)[4]) {
+                const float v[16] = {d[0].x, d[0].y, d[0].z, d[0].w, d[1].x, d[1].y, d[1].z, d[1].w,
+                                     d[2].x, d[2].y, d[2].z, d[2].w, d[3].x, d[3].y, d[3].z, d[3].w};
+                run_add<16>(v, p1, p2);
+            };
+            const int n32 = n / 32 * 32;
+            if (n32) ld(q0, 0);
+            for (; i < n32; i += 32) {  // the next 16 samples are loaded before these are added
+                ld(q1, i + 16);
+                add(q0);
+                if (i + 32 < n32) ld(q0, i + 32);
+                add(q1);
+            }
+        }
+        for (; i < n; ++i) {
+            const float v[1] = {p[i]};
+            run_add<1>(v, p1, p2);
+        }
+        part[q] = make_double2(p1, p2);
+    }
+    __syncthreads();
+    for (int r = tid; r < rows; r += kChanF32Threads) {
+        double s1 = 0.0, s2 = 0.0;
+        for (int j = 0; j < nruns; ++j) {
+            const double2 d = part[r * nruns + j];
+            s1 = __dadd_rn(s1, d.x);
+            s2 = __dadd_rn(s2, d.y);
+        }
+        clip[r] = float_clip(s1, s2, (double)len, k);
+    }
+    __syncthreads();
+    for (int r = 0; r < rows; ++r) {
+        float *row = x + (size_t)(c0 + r) * (size_t)stride;
+        const FloatClip c = clip[r];
+        auto bad = [&](float v) { return v <= c.lo || v >= c.hi; };
+        long long done = 0;
+        if (vec) {
+            const long long nv = len / 4;
+            done = nv * 4;
+#pragma unroll 4
+            for (long long i = tid; i < nv; i += kChanF32Threads) {
+                float4 *p = reinterpret_cast<float4 *>(row) + i;
+                float4 v = *p;
+                if (bad(v.x) || bad(v.y) || bad(v.z) || bad(v.w)) {
+                    v.x = bad(v.x) ? c.rep : v.x;
+                    v.y = bad(v.y) ? c.rep : v.y;
+                    v.z = bad(v.z) ? c.rep : v.z;
+                    v.w = bad(v.w) ? c.rep : v.w;
+                    *p = v;
+                }
+            }
+        }
+        for (long long i = done + tid; i < len; i += kChanF32Threads)
+            if (bad(row[i])) row[i] = c.rep;
+    }
+}
+
+constexpr int kSpecF32Rows = 8;  // threads per column
+
+// Spectra of float samples: 32 columns a CTA; a thread sums runs of 1024 channels of its column
+// left to right, one thread a column adds the runs left to right, then all threads clip.
+__global__ void __launch_bounds__(32 * kSpecF32Rows)
+    k_clip_spectra_f32(float *__restrict__ x, int nchans, long long stride, long long len, double k)
+{
+    __shared__ double2 part[kSpecF32Rows][32];
+    __shared__ FloatClip clip[32];
+    const int lane = threadIdx.x, ty = threadIdx.y;
+    const long long t = (long long)blockIdx.x * 32 + lane;
+    const bool in = t < len;
+    const int nruns = (nchans + kRun - 1) / kRun;
+    double s1 = 0.0, s2 = 0.0;  // (threads ty 0)
+    for (int r0 = 0; r0 < nruns; r0 += kSpecF32Rows) {
+        const int r = r0 + ty;
+        const int ca = r * kRun, cb = min(ca + kRun, nchans);
+        double p1 = 0.0, p2 = 0.0;
+        if (in && r < nruns) {
+            constexpr int U = 8;
+            const float *p = x + (size_t)ca * (size_t)stride + t;
+            int n = cb - ca;
+            float a[U], b[U];
+            auto ld = [&](float (&d)[U], int at) {
+#pragma unroll
+                for (int j = 0; j < U; ++j) d[j] = p[(size_t)(at + j) * (size_t)stride];
+            };
+            const int n16 = n / (2 * U) * (2 * U);
+            int i = 0;
+            if (n16) ld(a, 0);
+            for (; i < n16; i += 2 * U) {
+                ld(b, i + U);
+                run_add<U>(a, p1, p2);
+                if (i + 2 * U < n16) ld(a, i + 2 * U);
+                run_add<U>(b, p1, p2);
+            }
+            for (; i < n; ++i) {
+                const float v[1] = {p[(size_t)i * (size_t)stride]};
+                run_add<1>(v, p1, p2);
+            }
+        }
+        if (r0 > 0) __syncthreads();  // the previous runs are added
+        part[ty][lane] = make_double2(p1, p2);
+        __syncthreads();
+        if (ty == 0)
+            for (int j = 0; j < min(kSpecF32Rows, nruns - r0); ++j) {
+                s1 = __dadd_rn(s1, part[j][lane].x);
+                s2 = __dadd_rn(s2, part[j][lane].y);
+            }
+    }
+    if (ty == 0 && in) clip[lane] = float_clip(s1, s2, (double)nchans, k);
+    __syncthreads();
+    if (!in) return;
+    const FloatClip c = clip[lane];
+#pragma unroll 8
+    for (int ch = ty; ch < nchans; ch += kSpecF32Rows) {
+        float *p = x + (size_t)ch * (size_t)stride + t;
+        const float v = *p;
+        if (v <= c.lo || v >= c.hi) *p = c.rep;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// launches
+// ------------------------------------------------------------------------------------------
+template <typename T, int NV>
+mdsm_status launch_spectra_int(T *x, int nchans, long long stride, long long len, double ks,
+                               cudaStream_t st)
+{
+    constexpr int N = 16 / (int)sizeof(T);
+    const int per = kSpecThreads / 2 * NV;
+    const int ncl = std::min(8, (nchans + per - 1) / per);
+    const int nbatch = (nchans + per * ncl - 1) / (per * ncl);
+    const long long tiles = (len + 2 * N - 1) / (2 * N);
+    if (tiles * ncl > 0x7fffffffLL) return fail(MDSM_EINVAL, "rfi clip: block too long");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles * ncl));
+    cfg.blockDim = dim3(kSpecThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ncl;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    MDSM_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_clip_spectra_int<T, NV>, x, nchans, stride, len, ks,
+                                     nbatch));
+    return MDSM_OK;
+}
+
 template <typename T>
-static mdsm_status clip_t(T *x, int nchans, long long stride, long long len, double kc, double ks,
-                          cudaStream_t st)
+mdsm_status clip_int(T *x, int nchans, long long stride, long long len, double kc, double ks,
+                     cudaStream_t st)
 {
     if (kc > 0.0) {
-        size_t smem = 0;
-        if (!is_int_sample<T>()) {
-            smem = (size_t)((len + 1023) / 1024) * sizeof(double2);
-            if (smem > 200 * 1024) return fail(MDSM_EINVAL, "rfi clip: row too long");
-            MDSM_CUDA_TRY(cudaFuncSetAttribute(k_clip_channels<T>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem));
-        }
-        k_clip_channels<T><<<nchans, 256, smem, st>>>(x, stride, len, kc);
+        k_clip_channels_int<T><<<nchans, kChanThreads, 0, st>>>(x, stride, len, kc);
         MDSM_CUDA_TRY(cudaGetLastError());
     }
     if (ks > 0.0) {
-        k_clip_spectra<T><<<(unsigned)((len + 255) / 256), 256, 0, st>>>(x, nchans, stride, len, ks);
+        // the vector form where every row starts on a 16-byte boundary; few channels take two
+        // vectors a thread (512 channels a CTA) instead of eight
+        if ((((uintptr_t)x | (uintptr_t)(stride * (long long)sizeof(T))) & 15) == 0)
+            return nchans <= kSpecThreads ? launch_spectra_int<T, 2>(x, nchans, stride, len, ks, st)
+                                          : launch_spectra_int<T, 8>(x, nchans, stride, len, ks, st);
+        k_clip_spectra_any<T><<<(unsigned)((len + 255) / 256), 256, 0, st>>>(x, nchans, stride, len,
+                                                                             ks);
         MDSM_CUDA_TRY(cudaGetLastError());
     }
     return MDSM_OK;
 }
 
+mdsm_status clip_f32(float *x, int nchans, long long stride, long long len, double kc, double ks,
+                     cudaStream_t st)
+{
+    if (kc > 0.0) {
+        const long long nruns = (len + kRun - 1) / kRun;
+        if (nruns * (long long)sizeof(double2) > 200 * 1024)
+            return fail(MDSM_EINVAL, "rfi clip: row too long");
+        // rows a CTA: enough runs for its threads, while two CTAs a SM remain
+        const int rpc = (int)std::max<long long>(
+            1, std::min<long long>({kChanF32Threads / nruns, nchans / 304, kChanF32Threads}));
+        const size_t smem = (size_t)(rpc * nruns) * sizeof(double2);
+        MDSM_CUDA_TRY(cudaFuncSetAttribute(k_clip_channels_f32,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_clip_channels_f32<<<(nchans + rpc - 1) / rpc, kChanF32Threads, smem, st>>>(
+            x, nchans, stride, len, kc, rpc);
+        MDSM_CUDA_TRY(cudaGetLastError());
+    }
+    if (ks > 0.0) {
+        k_clip_spectra_f32<<<(unsigned)((len + 31) / 32), dim3(32, kSpecF32Rows), 0, st>>>(
+            x, nchans, stride, len, ks);
+        MDSM_CUDA_TRY(cudaGetLastError());
+    }
+    return MDSM_OK;
+}
+
+}  // namespace
+
 mdsm_status rfi_clip(void *d_x, int dtype, int nchans, long long stride, long long len,
                      double k_chan, double k_spec, cudaStream_t st)
 {
     switch (dtype) {
-    case MDSM_U8: return clip_t(static_cast<uint8_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
+    case MDSM_U8:
+        return clip_int(static_cast<uint8_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
     case MDSM_U16:
-        return clip_t(static_cast<uint16_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
+        return clip_int(static_cast<uint16_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
     case MDSM_I16:
-        return clip_t(static_cast<int16_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
-    case MDSM_F32: return clip_t(static_cast<float *>(d_x), nchans, stride, len, k_chan, k_spec, st);
+        return clip_int(static_cast<int16_t *>(d_x), nchans, stride, len, k_chan, k_spec, st);
+    case MDSM_F32:
+        return clip_f32(static_cast<float *>(d_x), nchans, stride, len, k_chan, k_spec, st);
     }
     return fail(MDSM_EINVAL, "rfi clip: unknown sample type");
 }
