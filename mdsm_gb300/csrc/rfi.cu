@@ -136,7 +136,7 @@ constexpr int kChanThreads = 512;
 // far below its size), so the DRAM traffic is one read plus the vectors that change.  On uint8
 // 4096 ch x 97921 this replaced one byte a thread and three double operations a sample.
 template <typename T>
-__global__ void __launch_bounds__(kChanThreads)
+__global__ void __launch_bounds__(kChanThreads, 4)
     k_clip_channels_int(T *__restrict__ x, long long stride, long long len, double k)
 {
     constexpr int N = 16 / (int)sizeof(T);
@@ -222,11 +222,21 @@ __global__ void __launch_bounds__(kChanThreads)
     WordClip<T> wc;
     const IntClip c4[4] = {c, c, c, c};
     wc.set(c4);
-#pragma unroll 4
-    for (long long i = tid; i < nv; i += kChanThreads) {
-        const uint4 v = vec[i];
-        const uint4 q = make_uint4(wc.apply(v.x), wc.apply(v.y), wc.apply(v.z), wc.apply(v.w));
-        if (((q.x ^ v.x) | (q.y ^ v.y) | (q.z ^ v.z) | (q.w ^ v.w)) != 0u) vec[i] = q;
+    // (the loads of a batch before its stores: a store orders the loads behind it)
+    constexpr int U = 4;
+    for (long long i0 = tid; i0 < nv; i0 += U * kChanThreads) {
+        uint4 v[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (i0 + j * kChanThreads < nv) v[j] = vec[i0 + j * kChanThreads];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            if (i0 + j * kChanThreads >= nv) break;
+            const uint4 q = make_uint4(wc.apply(v[j].x), wc.apply(v[j].y), wc.apply(v[j].z),
+                                       wc.apply(v[j].w));
+            if (((q.x ^ v[j].x) | (q.y ^ v[j].y) | (q.z ^ v[j].z) | (q.w ^ v[j].w)) != 0u)
+                vec[i0 + j * kChanThreads] = q;
+        }
     }
 }
 
@@ -251,10 +261,13 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     const int tid = threadIdx.x, half = tid & 1;
     const long long t0 = (long long)(blockIdx.x / nrank) * (2 * N) + half * N;
     const int ncol = (int)max(0LL, min((long long)N, len - t0));  // columns of this vector
-    __shared__ unsigned long long sum1[2 * N], sum2[2 * N];
+    constexpr int NWARP = kSpecThreads / 32;
+    __shared__ long long w1[NWARP][2 * N];              // each warp's column sums
+    __shared__ unsigned long long w2[NWARP][2 * N];
+    __shared__ long long sum1[8][2 * N];                // each CTA of the cluster's
+    __shared__ unsigned long long sum2[8][2 * N];
     __shared__ IntClip clip[2 * N];
-    if (tid < 2 * N) sum1[tid] = sum2[tid] = 0ull;
-    __syncthreads();
+    const int warp = tid >> 5;
 
     uint32_t v[NV][4];
     auto channel = [&](int b, int i) {
@@ -324,13 +337,13 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                     for (int e = 0; e < 4; ++e) s2[e] += __shfl_xor_sync(0xffffffffu, s2[e], o);
                 }
                 if ((tid & 31) < 2) {
-                    const int q = half * N + 4 * w;
-                    atomicAdd(&sum1[q], (unsigned long long)(p01 & 0xffffu));
-                    atomicAdd(&sum1[q + 1], (unsigned long long)(p01 >> 16));
-                    atomicAdd(&sum1[q + 2], (unsigned long long)(p23 & 0xffffu));
-                    atomicAdd(&sum1[q + 3], (unsigned long long)(p23 >> 16));
+                    const uint32_t s1[4] = {p01 & 0xffffu, p01 >> 16, p23 & 0xffffu, p23 >> 16};
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) atomicAdd(&sum2[q + e], (unsigned long long)s2[e]);
+                    for (int e = 0; e < 4; ++e) {
+                        const int q = half * N + 4 * w + e;
+                        w1[warp][q] = (b ? w1[warp][q] : 0) + s1[e];
+                        w2[warp][q] = (b ? w2[warp][q] : 0) + s2[e];
+                    }
                 }
             } else {
                 int s1[2] = {0, 0};
@@ -353,23 +366,38 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
                 if ((tid & 31) < 2)
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        atomicAdd(&sum1[half * N + 2 * w + e], (unsigned long long)(long long)s1[e]);
-                        atomicAdd(&sum2[half * N + 2 * w + e], s2[e]);
+                        const int q = half * N + 2 * w + e;
+                        w1[warp][q] = (b ? w1[warp][q] : 0) + s1[e];
+                        w2[warp][q] = (b ? w2[warp][q] : 0) + s2[e];
                     }
             }
         }
     }
     __syncthreads();
-    cl.sync();  // every CTA's sums are complete
     if (tid < 2 * N) {
-        unsigned long long s1 = 0, s2 = 0;
-        for (int r = 0; r < nrank; ++r) {
-            s1 += *cl.map_shared_rank(&sum1[tid], r);
-            s2 += *cl.map_shared_rank(&sum2[tid], r);
+        long long s1 = 0;
+        unsigned long long s2 = 0;
+#pragma unroll
+        for (int q = 0; q < NWARP; ++q) {
+            s1 += w1[q][tid];
+            s2 += w2[q][tid];
         }
-        clip[tid] = int_clip<T>((long long)s1, (long long)s2, nchans, k);
+        for (int r = 0; r < nrank; ++r) {  // to every CTA of the cluster
+            *cl.map_shared_rank(&sum1[rank][tid], r) = s1;
+            *cl.map_shared_rank(&sum2[rank][tid], r) = s2;
+        }
     }
-    cl.sync();  // no CTA leaves while another reads its sums; clip[] is visible to its own CTA
+    cl.sync();  // every CTA's sums have arrived (no CTA touches another's memory after this)
+    if (tid < 2 * N) {
+        long long s1 = 0;
+        unsigned long long s2 = 0;
+        for (int r = 0; r < nrank; ++r) {
+            s1 += sum1[r][tid];
+            s2 += sum2[r][tid];
+        }
+        clip[tid] = int_clip<T>(s1, (long long)s2, nchans, k);
+    }
+    __syncthreads();
     for (int b = 0; b < nbatch; ++b) {
         if (nbatch > 1) load(b);
         uint32_t changed = 0;
@@ -439,9 +467,9 @@ __device__ __forceinline__ uint32_t special_key(float x)
     return (__float_as_uint(x) & 0x7f800000u) - 0x00800000u;  // >= 0x7f000000: special
 }
 
-// p1 += v, p2 += v * v (v * v is exact in double: one rounding each, as dmul + dadd) over U
-// consecutive samples.
-template <int U>
+// p1 += v, p2 += v * v over consecutive samples (v * v is exact in double: one rounding each, as
+// dmul + dadd).
+template <bool kSum1, int U>
 __device__ __forceinline__ void run_add(const float (&v)[U], double &p1, double &p2)
 {
     uint32_t sp = 0;
@@ -451,17 +479,146 @@ __device__ __forceinline__ void run_add(const float (&v)[U], double &p1, double 
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             const double d = float_bits_double(__float_as_uint(v[j]));
-            p1 = __dadd_rn(p1, d);
+            if (kSum1) p1 = __dadd_rn(p1, d);
             p2 = __fma_rn(d, d, p2);
         }
     } else {
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             const double d = (double)v[j];
-            p1 = __dadd_rn(p1, d);
+            if (kSum1) p1 = __dadd_rn(p1, d);
             p2 = __fma_rn(d, d, p2);
         }
     }
+}
+
+// The sum of a run of at most 1024 floats, where the left-to-right double sum rounds nothing: a
+// float is cut at three fixed places, and each third is added exactly in float.  With E the
+// exponent of a typical large sample, the thirds are whole multiples of u1 = 2^(E-11), u2 =
+// 2^(E-26) and u3 = 2^(E-41); cutting with a constant C = 1.5 * 2^23 units rounds to the unit
+// (for a sample below 2^22 of the first), so the second and third hold at most half a unit of
+// the one before (1024 of them stay within 2^24 units: exact adds), and the first is watched.
+// What a rare small sample leaves past the third is added exactly beside them, and its lowest
+// bit noted.  While the first's sums stay below 2^23 u1 and 2^53 lowest bits, every partial sum
+// is a whole number of lowest bits below 2^53: the double sum is exact at every step, in any
+// order.  Otherwise (ok() false) the caller sums in double.  15 float operations a sample
+// against one at the double rate (64 clocks of a scheduler for a warp).
+struct CutSum {
+    float c1, c2, c3, a1, a2, a3, a4, left, seen, top, unit;
+    __device__ __forceinline__ void start(float biggest)
+    {
+        // 2^E as a float, 0 (no cut fits) for zero, tiny, huge or special values
+        const uint32_t e = __float_as_uint(biggest) & 0x7f800000u;
+        const float p = e > (100u << 23) && e < (160u << 23) ? __uint_as_float(e) : 0.0f;
+        c1 = p * 6144.0f;            // 1.5 * 2^(23 + E - 11)
+        c2 = p * (1.5f / 8.0f);      // 1.5 * 2^(23 + E - 26)
+        c3 = p * (1.5f / 262144.0f); // 1.5 * 2^(23 + E - 41)
+        unit = c3 * (1.0f / 12582912.0f);
+        a1 = a2 = a3 = a4 = left = seen = top = 0.0f;
+    }
+    // the thirds of x; returns what is left past them
+    __device__ __forceinline__ float cut(float x, float &h1, float &h2, float &h3) const
+    {
+        h1 = __fsub_rn(__fadd_rn(x, c1), c1);
+        const float r1 = __fsub_rn(x, h1);
+        h2 = __fsub_rn(__fadd_rn(r1, c2), c2);
+        const float r2 = __fsub_rn(r1, h2);
+        h3 = __fsub_rn(__fadd_rn(r2, c3), c3);
+        return __fsub_rn(r2, h3);
+    }
+    template <int U>
+    __device__ __forceinline__ void add(const float (&v)[U])
+    {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            float h1, h2, h3;
+            const float r3 = cut(v[j], h1, h2, h3);
+            a1 = __fadd_rn(a1, h1);
+            a2 = __fadd_rn(a2, h2);
+            a3 = __fadd_rn(a3, h3);
+            left = __fadd_rn(left, fabsf(r3));
+            top = fmaxf(top, fmaxf(fabsf(a1), __fadd_rn(fabsf(v[j]), fabsf(v[j]))));
+        }
+        if (left == seen) return;
+        // some sample of these left a part past the third (or is not finite: left turns NaN)
+#pragma unroll 1
+        for (int j = 0; j < U; ++j) {
+            float x = v[0];
+#pragma unroll
+            for (int q = 1; q < U; ++q) x = j == q ? v[q] : x;
+            float h1, h2, h3;
+            const float r3 = cut(x, h1, h2, h3);
+            if (r3 == 0.0f) continue;
+            const float s = __fadd_rn(a4, r3), bb = __fsub_rn(s, a4);
+            const float err = __fadd_rn(__fsub_rn(a4, __fsub_rn(s, bb)), __fsub_rn(r3, bb));
+            const uint32_t b = __float_as_uint(x), m = (b & 0x7fffffu) | 0x800000u;
+            // the lowest bit of x: 2^(e - 150) times the lowest set bit of its significand
+            const float low = __fmul_rn(__uint_as_float(b & 0x7f800000u),
+                                        __fmul_rn((float)(m & (0u - m)), 1.0f / 8388608.0f));
+            unit = err == 0.0f && low > 0.0f ? fminf(unit, low) : 0.0f;
+            a4 = s;
+        }
+        seen = left;
+    }
+    __device__ __forceinline__ bool ok() const
+    {
+        // (2^53 lowest bits as 2^29 of them times 2^24; NaN and infinities fail a comparison)
+        return c1 > 0.0f && left < INFINITY && top < c1 * 0.66f &&
+               top * (1.01f / 536870912.0f) < unit * 16777216.0f;
+    }
+    __device__ __forceinline__ double sum() const
+    {
+        return __dadd_rn(__dadd_rn(__dadd_rn((double)a1, (double)a2), (double)a3), (double)a4);
+    }
+};
+
+// Left-to-right double sums of n (at most 1024) samples and of their squares; ld(v, at) loads
+// samples [at, at + 16), one(at) a single one.
+template <class Ld, class One>
+__device__ __forceinline__ double2 run_sums(int n, const Ld &ld, const One &one)
+{
+    constexpr int U = 16;
+    double p1 = 0.0, p2 = 0.0;
+    CutSum cs;
+    float a[U], b[U];
+    const int n2 = n / (2 * U) * (2 * U);
+    float big = 0.0f;
+    if (n2) {
+        ld(a, 0);
+        // maxima of four samples, two by two the smaller, of these the larger: outliers among the
+        // first samples do not move it
+        float m[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            m[j] = fmaxf(fmaxf(fabsf(a[4 * j]), fabsf(a[4 * j + 1])),
+                         fmaxf(fabsf(a[4 * j + 2]), fabsf(a[4 * j + 3])));
+        big = fmaxf(fminf(m[0], m[1]), fminf(m[2], m[3]));
+    }
+    cs.start(big);
+    for (int i = 0; i < n2; i += 2 * U) {  // the next 16 samples are loaded before these are added
+        ld(b, i + U);
+        cs.add(a);
+        run_add<false, U>(a, p1, p2);
+        if (i + 2 * U < n2) ld(a, i + 2 * U);
+        cs.add(b);
+        run_add<false, U>(b, p1, p2);
+    }
+    for (int i = n2; i < n; ++i) {
+        const float v[1] = {one(i)};
+        cs.add(v);
+        run_add<false, 1>(v, p1, p2);
+    }
+    if (cs.ok()) return make_double2(cs.sum(), p2);
+    for (int i = 0; i < n2; i += U) {
+        ld(a, i);
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            p1 = __dadd_rn(p1, special_key(a[j]) < 0x7f000000u
+                                   ? float_bits_double(__float_as_uint(a[j]))
+                                   : (double)a[j]);
+    }
+    for (int i = n2; i < n; ++i) p1 = __dadd_rn(p1, (double)one(i));
+    return make_double2(p1, p2);
 }
 
 struct FloatClip {
@@ -479,18 +636,19 @@ __device__ __forceinline__ FloatClip float_clip(double s1, double s2, double n, 
     return c;
 }
 
-constexpr int kChanF32Threads = 128;
+constexpr int kChanF32Threads = 256;
+constexpr int kChanF32Runs = 128;  // runs of a CTA's rows that the row count aims at
 
 // Channels of float samples: a CTA takes `rpc` rows, one thread per run of 1024 samples of a
 // row (left to right), then the runs' sums left to right, then the clip in float.  Several rows
 // a CTA because a warp of double operations costs the same with few lanes as with 32.
-__global__ void __launch_bounds__(kChanF32Threads)
+__global__ void __launch_bounds__(kChanF32Threads, 3)
     k_clip_channels_f32(float *__restrict__ x, int nchans, long long stride, long long len,
                         double k, int rpc)
 {
     extern __shared__ __align__(16) unsigned char sm[];
     double2 *part = reinterpret_cast<double2 *>(sm);  // [rpc][nruns]
-    __shared__ FloatClip clip[kChanF32Threads];
+    __shared__ FloatClip clip[kChanF32Runs];
     const int tid = threadIdx.x;
     const int c0 = blockIdx.x * rpc, rows = min(rpc, nchans - c0);
     const int nruns = (int)((len + kRun - 1) / kRun);
@@ -500,33 +658,29 @@ __global__ void __launch_bounds__(kChanF32Threads)
         const long long i0 = (long long)(q - r * nruns) * kRun;
         const float *p = x + (size_t)(c0 + r) * (size_t)stride + i0;
         const int n = (int)min((long long)kRun, len - i0);
-        double p1 = 0.0, p2 = 0.0;
-        int i = 0;
-        if (vec) {
-            float4 q0[4], q1[4];
-            auto ld = [&](float4 (&d)[4], int at) {
+        auto one = [&](int i) { return p[i]; };
+        if (vec)
+            part[q] = run_sums(
+                n,
+                [&](float (&d)[16], int at) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) d[j] = *reinterpret_cast<const float4 *>(p + at + 4 * j);
-            };
-            auto add = [&](const float4 (&d)[4]) {
-                const float v[16] = {d[0].x, d[0].y, d[0].z, d[0].w, d[1].x, d[1].y, d[1].z, d[1].w,
-                                     d[2].x, d[2].y, d[2].z, d[2].w, d[3].x, d[3].y, d[3].z, d[3].w};
-                run_add<16>(v, p1, p2);
-            };
-            const int n32 = n / 32 * 32;
-            if (n32) ld(q0, 0);
-            for (; i < n32; i += 32) {  // the next 16 samples are loaded before these are added
-                ld(q1, i + 16);
-                add(q0);
-                if (i + 32 < n32) ld(q0, i + 32);
-                add(q1);
-            }
-        }
-        for (; i < n; ++i) {
-            const float v[1] = {p[i]};
-            run_add<1>(v, p1, p2);
-        }
-        part[q] = make_double2(p1, p2);
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 u = *reinterpret_cast<const float4 *>(p + at + 4 * j);
+                        d[4 * j] = u.x;
+                        d[4 * j + 1] = u.y;
+                        d[4 * j + 2] = u.z;
+                        d[4 * j + 3] = u.w;
+                    }
+                },
+                one);
+        else
+            part[q] = run_sums(
+                n,
+                [&](float (&d)[16], int at) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) d[j] = p[at + j];
+                },
+                one);
     }
     __syncthreads();
     for (int r = tid; r < rows; r += kChanF32Threads) {
@@ -547,16 +701,25 @@ __global__ void __launch_bounds__(kChanF32Threads)
         if (vec) {
             const long long nv = len / 4;
             done = nv * 4;
-#pragma unroll 4
-            for (long long i = tid; i < nv; i += kChanF32Threads) {
-                float4 *p = reinterpret_cast<float4 *>(row) + i;
-                float4 v = *p;
-                if (bad(v.x) || bad(v.y) || bad(v.z) || bad(v.w)) {
-                    v.x = bad(v.x) ? c.rep : v.x;
-                    v.y = bad(v.y) ? c.rep : v.y;
-                    v.z = bad(v.z) ? c.rep : v.z;
-                    v.w = bad(v.w) ? c.rep : v.w;
-                    *p = v;
+            // (the loads of a batch before its stores: a store orders the loads behind it)
+            constexpr int U = 4;
+            float4 *rv = reinterpret_cast<float4 *>(row);
+            for (long long i0 = tid; i0 < nv; i0 += U * kChanF32Threads) {
+                float4 v[U];
+#pragma unroll
+                for (int j = 0; j < U; ++j)
+                    if (i0 + j * kChanF32Threads < nv) v[j] = rv[i0 + j * kChanF32Threads];
+#pragma unroll
+                for (int j = 0; j < U; ++j) {
+                    if (i0 + j * kChanF32Threads >= nv) break;
+                    float4 &q = v[j];
+                    if (bad(q.x) || bad(q.y) || bad(q.z) || bad(q.w)) {
+                        q.x = bad(q.x) ? c.rep : q.x;
+                        q.y = bad(q.y) ? c.rep : q.y;
+                        q.z = bad(q.z) ? c.rep : q.z;
+                        q.w = bad(q.w) ? c.rep : q.w;
+                        rv[i0 + j * kChanF32Threads] = q;
+                    }
                 }
             }
         }
@@ -565,52 +728,44 @@ __global__ void __launch_bounds__(kChanF32Threads)
     }
 }
 
-constexpr int kSpecF32Rows = 8;  // threads per column
+constexpr int kSpecF32Threads = 256;
 
-// Spectra of float samples: 32 columns a CTA; a thread sums runs of 1024 channels of its column
-// left to right, one thread a column adds the runs left to right, then all threads clip.
-__global__ void __launch_bounds__(32 * kSpecF32Rows)
+// Spectra of float samples: COLS columns a CTA, kSpecF32Threads / COLS threads a column; a thread
+// sums runs of 1024 channels of its column left to right, one thread a column adds the runs left
+// to right, then all threads clip.  128 columns where that leaves two CTAs a SM: the four warps
+// that sum then lie on the SM's four schedulers, each with its own double unit; 32 columns
+// otherwise.
+template <int COLS>
+__global__ void __launch_bounds__(kSpecF32Threads)
     k_clip_spectra_f32(float *__restrict__ x, int nchans, long long stride, long long len, double k)
 {
-    __shared__ double2 part[kSpecF32Rows][32];
-    __shared__ FloatClip clip[32];
+    constexpr int kRows = kSpecF32Threads / COLS;
+    __shared__ double2 part[kRows][COLS];
+    __shared__ FloatClip clip[COLS];
     const int lane = threadIdx.x, ty = threadIdx.y;
-    const long long t = (long long)blockIdx.x * 32 + lane;
+    const long long t = (long long)blockIdx.x * COLS + lane;
     const bool in = t < len;
     const int nruns = (nchans + kRun - 1) / kRun;
     double s1 = 0.0, s2 = 0.0;  // (threads ty 0)
-    for (int r0 = 0; r0 < nruns; r0 += kSpecF32Rows) {
+    for (int r0 = 0; r0 < nruns; r0 += kRows) {
         const int r = r0 + ty;
         const int ca = r * kRun, cb = min(ca + kRun, nchans);
-        double p1 = 0.0, p2 = 0.0;
+        double2 sums = make_double2(0.0, 0.0);
         if (in && r < nruns) {
-            constexpr int U = 8;
             const float *p = x + (size_t)ca * (size_t)stride + t;
-            int n = cb - ca;
-            float a[U], b[U];
-            auto ld = [&](float (&d)[U], int at) {
+            sums = run_sums(
+                cb - ca,
+                [&](float (&d)[16], int at) {
 #pragma unroll
-                for (int j = 0; j < U; ++j) d[j] = p[(size_t)(at + j) * (size_t)stride];
-            };
-            const int n16 = n / (2 * U) * (2 * U);
-            int i = 0;
-            if (n16) ld(a, 0);
-            for (; i < n16; i += 2 * U) {
-                ld(b, i + U);
-                run_add<U>(a, p1, p2);
-                if (i + 2 * U < n16) ld(a, i + 2 * U);
-                run_add<U>(b, p1, p2);
-            }
-            for (; i < n; ++i) {
-                const float v[1] = {p[(size_t)i * (size_t)stride]};
-                run_add<1>(v, p1, p2);
-            }
+                    for (int j = 0; j < 16; ++j) d[j] = p[(size_t)(at + j) * (size_t)stride];
+                },
+                [&](int i) { return p[(size_t)i * (size_t)stride]; });
         }
         if (r0 > 0) __syncthreads();  // the previous runs are added
-        part[ty][lane] = make_double2(p1, p2);
+        part[ty][lane] = sums;
         __syncthreads();
         if (ty == 0)
-            for (int j = 0; j < min(kSpecF32Rows, nruns - r0); ++j) {
+            for (int j = 0; j < min(kRows, nruns - r0); ++j) {
                 s1 = __dadd_rn(s1, part[j][lane].x);
                 s2 = __dadd_rn(s2, part[j][lane].y);
             }
@@ -619,11 +774,16 @@ __global__ void __launch_bounds__(32 * kSpecF32Rows)
     __syncthreads();
     if (!in) return;
     const FloatClip c = clip[lane];
-#pragma unroll 8
-    for (int ch = ty; ch < nchans; ch += kSpecF32Rows) {
+    constexpr int U = 16;
+    for (int ch = ty; ch < nchans; ch += U * kRows) {
         float *p = x + (size_t)ch * (size_t)stride + t;
-        const float v = *p;
-        if (v <= c.lo || v >= c.hi) *p = c.rep;
+        const size_t step = (size_t)kRows * (size_t)stride;
+        float v[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) v[j] = ch + j * kRows < nchans ? p[j * step] : c.rep;
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+            if (ch + j * kRows < nchans && (v[j] <= c.lo || v[j] >= c.hi)) p[j * step] = c.rep;
     }
 }
 
@@ -685,8 +845,9 @@ mdsm_status clip_f32(float *x, int nchans, long long stride, long long len, doub
             return fail(MDSM_EINVAL, "rfi clip: row too long");
         // rows a CTA: enough runs for its threads, while two CTAs a SM remain
         const int rpc = (int)std::max<long long>(
-            1, std::min<long long>({kChanF32Threads / nruns, nchans / 304, kChanF32Threads}));
-        const size_t smem = (size_t)(rpc * nruns) * sizeof(double2);
+            1, std::min<long long>({kChanF32Runs / nruns, (nchans + 303) / 304}));
+        // (close to a third of a SM's shared memory: at most three CTAs share its double units)
+        const size_t smem = std::max<size_t>((size_t)(rpc * nruns) * sizeof(double2), 72 * 1024);
         MDSM_CUDA_TRY(cudaFuncSetAttribute(k_clip_channels_f32,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_clip_channels_f32<<<(nchans + rpc - 1) / rpc, kChanF32Threads, smem, st>>>(
@@ -694,8 +855,14 @@ mdsm_status clip_f32(float *x, int nchans, long long stride, long long len, doub
         MDSM_CUDA_TRY(cudaGetLastError());
     }
     if (ks > 0.0) {
-        k_clip_spectra_f32<<<(unsigned)((len + 31) / 32), dim3(32, kSpecF32Rows), 0, st>>>(
-            x, nchans, stride, len, ks);
+        if (len >= 304 * 128)
+            k_clip_spectra_f32<128>
+                <<<(unsigned)((len + 127) / 128), dim3(128, kSpecF32Threads / 128), 0, st>>>(
+                    x, nchans, stride, len, ks);
+        else
+            k_clip_spectra_f32<32>
+                <<<(unsigned)((len + 31) / 32), dim3(32, kSpecF32Threads / 32), 0, st>>>(
+                    x, nchans, stride, len, ks);
         MDSM_CUDA_TRY(cudaGetLastError());
     }
     return MDSM_OK;
