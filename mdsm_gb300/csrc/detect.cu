@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "box.cuh"
+#include "cutsum.cuh"
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -78,47 +79,377 @@ __device__ __forceinline__ float median5(float n1, float n2, float n3, float n4,
     return (d < a) ? d : a;
 }
 
-// One thread per 32K chunk: sequential double sums (dedispersion_output.cpp:155-160).
-__global__ void k_ref_chunk_sums(const float *__restrict__ buf, unsigned mod, unsigned nchunks,
-                                 double2 *__restrict__ sums)
+// ---------------------------------------------------------------------------------------------
+// Block statistics (dedispersion_output.cpp:154-168): per 32768-value chunk the left-to-right
+// double sums t1 and t2 of the values and of their squares; over the chunks, in float,
+// localmean = localmean + t1 / mod, and in double mean2 += t2 / mod; then
+// mean = localmean / nchunks and rms = sqrt(mean2 / nchunks - mean * mean), both floats.
+//
+// Summed as written, a chunk is a chain of 32768 steps of two double operations, 64 clocks each:
+// 2 ms whatever the block's size.  So the sums are first formed in parallel (k_ref_chunk_fast):
+// t1 exactly, with the largest |partial sum| bounded, which tells whether the chain rounds at all
+// and bounds its error where it does; t2 to 2^-36 of itself, which also covers its chain.
+// k_ref_finish_fast forms mean and rms from them and checks that nothing within those bounds
+// would round to other floats.  Where it would (or the values do not suit the exact sum), it
+// raises *redo, and the chains run as written (k_ref_chunk_seq, k_ref_finish_seq); otherwise those
+// two return at once.  Zero-mean float series of 2^26 values: 5.8 ms as chains of one thread a
+// chunk, now 0.1 ms.
+// ---------------------------------------------------------------------------------------------
+constexpr int kRefThreads = 256;
+constexpr int kRefBatch = 512;   // values of one warp's batch (16 a lane)
+constexpr float kRefRel = 1.0f / 68719476736.0f;  // 2^-36
+
+struct RefChunk {
+    double d, m2;  // t1 / mod, t2 / mod
+};
+
+// One CTA a chunk; eps: a bound on how far t1 / mod may be from the chain's (infinite: unknown).
+__global__ void __launch_bounds__(kRefThreads)
+    k_ref_chunk_fast(const float *__restrict__ buf, unsigned mod, RefChunk *__restrict__ out,
+                     float *__restrict__ eps)
 {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nchunks) return;
-    const float *p = buf + (size_t)i * mod;
-    double t1 = 0.0, t2 = 0.0;
-    for (unsigned j = 0; j < mod; ++j) {
-        const double v = (double)__ldg(p + j);
-        t1 = __dadd_rn(t1, v);
-        t2 = __fma_rn(v, v, t2);  // v*v exact: same as dmul + dadd
+    constexpr int NW = kRefThreads / 32, U = 16;
+    __shared__ float s_sum[128], s_abs[128];  // batch sums in order: 8 warps x at most 16
+    __shared__ float w_anchor[NW], w_unit[NW];
+    __shared__ long long w_i[3][NW];
+    __shared__ double w_a4[NW], w_t2[NW];
+    __shared__ int w_ok[NW];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const float *p = buf + (size_t)blockIdx.x * mod;
+    const bool vec = (((uintptr_t)p) & 15) == 0;
+    // each warp a run of whole batches
+    const unsigned nbat = (mod + kRefBatch - 1) / kRefBatch, per = (nbat + NW - 1) / NW;
+    auto load = [&](float (&v)[U], unsigned bat) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const unsigned i = bat * kRefBatch + k * 128 + lane * 4;
+            if (vec && i + 3 < mod) {
+                const float4 q = __ldg(reinterpret_cast<const float4 *>(p + i));
+                v[4 * k] = q.x;
+                v[4 * k + 1] = q.y;
+                v[4 * k + 2] = q.z;
+                v[4 * k + 3] = q.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[4 * k + e] = i + e < mod ? __ldg(p + i + e) : 0.0f;
+            }
+        }
+    };
+    // one cut for the whole chunk, placed by the mean magnitude of some of its values
+    {
+        const unsigned stride = max(1u, mod / kRefThreads);
+        float a = tid * stride < mod ? fabsf(__ldg(p + tid * stride)) : 0.0f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) w_anchor[warp] = a;
     }
-    sums[i] = make_double2(t1, t2);
+    __syncthreads();
+    float anchor = 0.0f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) anchor = fmaxf(anchor, w_anchor[w] * (1.0f / 16.0f));
+    CutSum cs;
+    cs.start(anchor);
+    const float u1 = cs.c1 * (1.0f / 12582912.0f), u2 = cs.c2 * (1.0f / 12582912.0f),
+                u3 = cs.c3 * (1.0f / 12582912.0f);
+    double t2 = 0.0;
+    float s = 0.0f, c = 0.0f;  // squares: a compensated float sum, folded into t2 every 32
+    float v[U], nx[U];
+    const unsigned b0 = warp * per, b1 = min(nbat, b0 + per);
+    if (b0 < b1) load(v, b0);
+    for (unsigned b = b0; b < b1; ++b) {
+        if (b + 1 < b1) load(nx, b + 1);
+        cs.add(v);
+        float bs = 0.0f, ba = 0.0f;
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            bs += v[j];
+            ba += fabsf(v[j]);
+            const float q = __fmul_rn(v[j], v[j]), e = __fmaf_rn(v[j], v[j], -q);
+            const float n = __fadd_rn(s, q), bb = __fsub_rn(n, s);
+            c = __fadd_rn(c, __fadd_rn(__fadd_rn(__fsub_rn(s, __fsub_rn(n, bb)), __fsub_rn(q, bb)), e));
+            s = n;
+        }
+        if (((b - b0) & 1u) || b + 1 == b1) {
+            t2 = __dadd_rn(t2, __dadd_rn((double)s, (double)c));
+            s = c = 0.0f;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            bs += __shfl_xor_sync(0xffffffffu, bs, o);
+            ba += __shfl_xor_sync(0xffffffffu, ba, o);
+        }
+        if (lane == 0) {
+            s_sum[b] = bs;
+            s_abs[b] = ba;
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) v[j] = nx[j];
+    }
+    // the warps' sums: the thirds as whole numbers of their units
+    long long i1 = 0, i2 = 0, i3 = 0;
+    const bool ok = cs.c1 > 0.0f && cs.left < INFINITY && cs.top < cs.c1 * 0.66f;
+    if (ok) {
+        i1 = __float2ll_rn(cs.a1 / u1);
+        i2 = __float2ll_rn(cs.a2 / u2);
+        i3 = __float2ll_rn(cs.a3 / u3);
+    }
+    double a4 = (double)cs.a4;
+    float unit = cs.unit;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        i1 += __shfl_xor_sync(0xffffffffu, i1, o);
+        i2 += __shfl_xor_sync(0xffffffffu, i2, o);
+        i3 += __shfl_xor_sync(0xffffffffu, i3, o);
+        a4 = __dadd_rn(a4, __shfl_xor_sync(0xffffffffu, a4, o));
+        t2 = __dadd_rn(t2, __shfl_xor_sync(0xffffffffu, t2, o));
+        unit = fminf(unit, __shfl_xor_sync(0xffffffffu, unit, o));
+    }
+    const bool allok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) {
+        w_i[0][warp] = i1;
+        w_i[1][warp] = i2;
+        w_i[2][warp] = i3;
+        w_a4[warp] = a4;
+        w_t2[warp] = t2;
+        w_unit[warp] = unit;
+        w_ok[warp] = allok;
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    // prefix sums at the batch boundaries bound every partial sum of the chain
+    float run = 0.0f, top = 0.0f, most = 0.0f, total = 0.0f;
+    for (unsigned k0 = 0; k0 < nbat; k0 += 32) {
+        const unsigned k = k0 + lane;
+        float x = k < nbat ? s_sum[k] : 0.0f;
+        const float a = k < nbat ? s_abs[k] : 0.0f;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        x += run;
+        top = fmaxf(top, fabsf(x));
+        most = fmaxf(most, a);
+        total += a;
+        run = __shfl_sync(0xffffffffu, x, 31);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+    }
+    if (lane != 0) return;
+    // (the batch sums are floats: their errors stay below 2^-14 of the sum of magnitudes)
+    const float m = 1.01f * (top + most) + total * (1.0f / 16384.0f);
+    bool good = true;
+    unit = INFINITY;
+    i1 = i2 = i3 = 0;
+    a4 = t2 = 0.0;
+    for (int w = 0; w < NW; ++w) {
+        good = good && w_ok[w];
+        unit = fminf(unit, w_unit[w]);
+        i1 += w_i[0][w];
+        i2 += w_i[1][w];
+        i3 += w_i[2][w];
+        a4 = __dadd_rn(a4, w_a4[w]);
+        t2 = __dadd_rn(t2, w_t2[w]);
+    }
+    const double t1 = __dadd_rn(
+        __dadd_rn(__dadd_rn(__dmul_rn((double)i1, (double)u1), __dmul_rn((double)i2, (double)u2)),
+                  __dmul_rn((double)i3, (double)u3)),
+        a4);
+    // every partial sum a whole number of the lowest bit and below 2^53 of them: no rounding in
+    // the chain; else at most 2^-53 of the largest in each of its mod steps
+    const bool exact = unit > 0.0f && m * (1.0f / 536870912.0f) < unit * 16777216.0f;
+    RefChunk r;
+    r.d = __ddiv_rn(t1, (double)mod);
+    r.m2 = __ddiv_rn(t2, (double)mod);
+    out[blockIdx.x] = r;
+    good = good && m < 1e30f && t2 < 1e30 && t2 > 1e-25;
+    eps[blockIdx.x] = !good ? INFINITY : exact ? 0.0f : m * (1.02f / 4503599627370496.0f);
 }
 
-// One thread: dedispersion_output.cpp:161-168.
-__global__ void k_ref_finish(const double2 *__restrict__ sums, unsigned mod, unsigned nchunks,
-                             float *__restrict__ stats)
+// l + d in double, then float, as float operations: s + e is l + dh exactly, dh + dl is d to
+// 2^-48 of itself.
+__device__ __forceinline__ void ref_step(float l, float dh, float dl, float &s, float &rest)
 {
+    s = __fadd_rn(l, dh);
+    const float bb = __fsub_rn(s, l);
+    const float e = __fadd_rn(__fsub_rn(l, __fsub_rn(s, bb)), __fsub_rn(dh, bb));
+    rest = __fadd_rn(e, dl);
+}
+
+__global__ void __launch_bounds__(kRefThreads)
+    k_ref_finish_fast(const RefChunk *__restrict__ ch, const float *__restrict__ eps,
+                      unsigned nchunks, float *__restrict__ stats, unsigned *__restrict__ redo)
+{
+    constexpr unsigned TILE = 2048;
+    __shared__ float dh[TILE], dl[TILE], lm[TILE + 1];
+    __shared__ double w_m2[kRefThreads / 32];
+    const int tid = threadIdx.x;
+    double m2 = 0.0;
+    bool bad = false;
+    float l = 0.0f;
+    for (unsigned k0 = 0; k0 < nchunks; k0 += TILE) {
+        const unsigned n = min(TILE, nchunks - k0);
+        __syncthreads();
+        for (unsigned i = tid; i < n; i += kRefThreads) {
+            const RefChunk r = ch[k0 + i];
+            m2 = __dadd_rn(m2, r.m2);
+            const float h = __double2float_rn(r.d);
+            dh[i] = h;
+            dl[i] = __double2float_rn(__dadd_rn(r.d, -(double)h));
+        }
+        __syncthreads();
+        if (tid == 0) {  // the chain: every step rounds the running mean to float
+#pragma unroll 8
+            for (unsigned i = 0; i < n; ++i) {
+                lm[i] = l;
+                float s, rest;
+                ref_step(l, dh[i], dl[i], s, rest);
+                l = __fadd_rn(s, rest);
+            }
+            lm[n] = l;
+        }
+        __syncthreads();
+        // every step again: no value within the bounds rounds to another float
+        for (unsigned i = tid; i < n; i += kRefThreads) {
+            float s, rest;
+            ref_step(lm[i], dh[i], dl[i], s, rest);
+            const float del = eps[k0 + i] * 1.01f +
+                              (fabsf(s) + fabsf(dh[i])) * (1.0f / 17592186044416.0f);  // 2^-44
+            const float a = __fadd_rn(s, __fadd_rn(rest, del)), b = __fadd_rn(s, __fadd_rn(rest, -del));
+            bad |= !(a == lm[i + 1] && b == lm[i + 1]);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m2 = __dadd_rn(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    if ((tid & 31) == 0) w_m2[tid >> 5] = m2;
+    const bool any = __syncthreads_or(bad) != 0;
+    if (tid != 0) return;
+    m2 = 0.0;
+    for (int w = 0; w < kRefThreads / 32; ++w) m2 = __dadd_rn(m2, w_m2[w]);
+    const float mean = __fdiv_rn(l, (float)nchunks);
+    const double sq = (double)__fmul_rn(mean, mean), q = __ddiv_rn(m2, (double)nchunks);
+    const double del = q * (double)kRefRel;
+    const float lo = __double2float_rn(__dsqrt_rn(__dadd_rn(__dadd_rn(q, -del), -sq)));
+    const float hi = __double2float_rn(__dsqrt_rn(__dadd_rn(__dadd_rn(q, del), -sq)));
+    stats[0] = mean;
+    stats[1] = lo;
+    *redo = !any && lo == hi ? 0u : 1u;
+}
+
+// The chains as written: a warp takes four chunks, its lanes stage 128 values of each in shared
+// memory, four lanes add them left to right.
+constexpr int kRefSeq = 4;
+__global__ void __launch_bounds__(32)
+    k_ref_chunk_seq(const float *__restrict__ buf, unsigned mod, unsigned nchunks,
+                    const unsigned *__restrict__ redo, RefChunk *__restrict__ out)
+{
+    if (*redo == 0u) return;
+    constexpr int N = 128;
+    __shared__ float st[kRefSeq][N + 1];
+    const int lane = threadIdx.x;
+    const unsigned c0 = blockIdx.x * kRefSeq;
+    float v[kRefSeq][4];
+    auto load = [&](unsigned i0) {
+#pragma unroll
+        for (int c = 0; c < kRefSeq; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const unsigned i = i0 + 32 * e + lane;
+                v[c][e] = c0 + c < nchunks && i < mod
+                              ? __ldg(buf + (size_t)(c0 + c) * mod + i) : 0.0f;
+            }
+    };
+    double t1 = 0.0, t2 = 0.0;
+    load(0);
+    for (unsigned i0 = 0; i0 < mod; i0 += N) {
+#pragma unroll
+        for (int c = 0; c < kRefSeq; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) st[c][32 * e + lane] = v[c][e];
+        __syncwarp();
+        if (i0 + N < mod) load(i0 + N);
+        if (lane < kRefSeq) {
+            const int n = (int)min((unsigned)N, mod - i0);
+#pragma unroll 8
+            for (int j = 0; j < n; ++j) {
+                const float x = st[lane][j];
+                const double d = special_key(x) < 0x7f000000u
+                                     ? float_bits_double(__float_as_uint(x)) : (double)x;
+                t1 = __dadd_rn(t1, d);
+                t2 = __fma_rn(d, d, t2);  // d*d exact: same as dmul + dadd
+            }
+        }
+        __syncwarp();
+    }
+    if (lane < kRefSeq && c0 + lane < nchunks) {
+        RefChunk r;
+        r.d = __ddiv_rn(t1, (double)mod);
+        r.m2 = __ddiv_rn(t2, (double)mod);
+        out[c0 + lane] = r;
+    }
+}
+
+// dedispersion_output.cpp:161-168, the running sums as written.
+__global__ void __launch_bounds__(kRefThreads)
+    k_ref_finish_seq(const RefChunk *__restrict__ ch, unsigned nchunks,
+                     const unsigned *__restrict__ redo, float *__restrict__ stats)
+{
+    if (*redo == 0u) return;
+    constexpr unsigned TILE = 1024;
+    __shared__ RefChunk t[TILE];
     float localmean = 0.0f;
     double mean2 = 0.0;
-    for (unsigned i = 0; i < nchunks; ++i) {
-        const double2 s = sums[i];
-        localmean = __double2float_rn(__dadd_rn((double)localmean, __ddiv_rn(s.x, (double)mod)));
-        mean2 = __dadd_rn(mean2, __ddiv_rn(s.y, (double)mod));
+    for (unsigned k0 = 0; k0 < nchunks; k0 += TILE) {
+        const unsigned n = min(TILE, nchunks - k0);
+        __syncthreads();
+        for (unsigned i = threadIdx.x; i < n; i += kRefThreads) t[i] = ch[k0 + i];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (unsigned i = 0; i < n; ++i)
+                localmean = __double2float_rn(__dadd_rn((double)localmean, t[i].d));
+        if (threadIdx.x == 32)
+            for (unsigned i = 0; i < n; ++i) mean2 = __dadd_rn(mean2, t[i].m2);
     }
+    __shared__ double s_m2;
+    if (threadIdx.x == 32) s_m2 = mean2;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
     localmean = __fdiv_rn(localmean, (float)nchunks);
     const float sq = __fmul_rn(localmean, localmean);
-    const double v = __dadd_rn(__ddiv_rn(mean2, (double)nchunks), -(double)sq);
+    const double v = __dadd_rn(__ddiv_rn(s_m2, (double)nchunks), -(double)sq);
     stats[0] = localmean;
     stats[1] = __double2float_rn(__dsqrt_rn(v));
+}
+
+// The block statistics of nchunks chunks of mod values: stats {mean, rms}; ch and eps: one entry
+// a chunk; redo: one word.
+static mdsm_status ref_stats(const float *d_series, unsigned mod, unsigned nchunks, RefChunk *ch,
+                             float *eps, unsigned *redo, float *stats, cudaStream_t st)
+{
+    k_ref_chunk_fast<<<nchunks, kRefThreads, 0, st>>>(d_series, mod, ch, eps);
+    k_ref_finish_fast<<<1, kRefThreads, 0, st>>>(ch, eps, nchunks, stats, redo);
+    k_ref_chunk_seq<<<(nchunks + kRefSeq - 1) / kRefSeq, 32, 0, st>>>(d_series, mod, nchunks, redo,
+                                                                      ch);
+    k_ref_finish_seq<<<1, kRefThreads, 0, st>>>(ch, nchunks, redo, stats);
+    MDSM_CUDA_TRY(cudaGetLastError());
+    return MDSM_OK;
 }
 
 // dedispersion_output.cpp:176-210 (mean == NULL).  Rows are the worker threads' rows in turn,
 // rpt per thread; row k of thread t has DM lowdm + (unsigned)(tshift * t) + k dmstep in float,
 // left to right (:187,194; one thread: rpt = ndms, tshift = 0).
-__global__ void k_ref_detect(const float *__restrict__ buf, int ndms, int nsamp, float lowdm,
-                             float dmstep, float threshold, const float *__restrict__ stats,
-                             DevCand *__restrict__ cands, unsigned long long *__restrict__ count,
-                             long long cap, int rpt, int tshift)
+//
+// A thread takes four window starts and reads its four samples once; the median is one of the
+// window's samples, so a window in which no sample passes the test (a NaN counts as passing)
+// cannot pass, and only the others' medians are formed.
+__global__ void __launch_bounds__(256)
+    k_ref_detect(const float *__restrict__ buf, int ndms, int nsamp, float lowdm, float dmstep,
+                 float threshold, const float *__restrict__ stats, DevCand *__restrict__ cands,
+                 unsigned long long *__restrict__ count, long long cap, int rpt, int tshift)
 {
     const int row = blockIdx.y;
     const unsigned t = (unsigned)row / (unsigned)rpt, k = (unsigned)row % (unsigned)rpt;
@@ -128,13 +459,36 @@ __global__ void k_ref_detect(const float *__restrict__ buf, int ndms, int nsamp,
     const float mean = stats[0], rms = stats[1];
     const float lim = __fmul_rn(rms, threshold);
     const float *r = buf + (size_t)row * nsamp;
-    const unsigned nl = (unsigned)nsamp - 4u;
-    for (unsigned l = blockIdx.x * blockDim.x + threadIdx.x; l < nl; l += gridDim.x * blockDim.x) {
-        const float m = median5(__ldg(r + l), __ldg(r + l + 1), __ldg(r + l + 2), __ldg(r + l + 3),
-                                __ldg(r + l + 4));
-        if (__fsub_rn(m, mean) >= lim) {
-            const unsigned long long at = atomicAdd(count, 1ull);
-            if ((long long)at < cap) cands[at] = DevCand{row, (int32_t)l, 1, __fdiv_rn(m, rms)};
+    const bool vec = (((uintptr_t)r) & 15) == 0;
+    const unsigned n = (unsigned)nsamp, nl = n - 4u;
+    auto may = [&](float v) { return !(__fsub_rn(v, mean) < lim); };
+    const int lane = threadIdx.x & 31;
+    // (whole warps run every iteration: the loop bound is the warp's)
+    for (unsigned l0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * 4u; l0 < nl;
+         l0 += gridDim.x * blockDim.x * 4u) {
+        const unsigned l = l0 + 4u * (unsigned)lane;
+        bool p = false;
+        if (vec && l + 3 < n) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(r + l));
+            p = may(q.x) || may(q.y) || may(q.z) || may(q.w);
+        } else {
+            for (unsigned e = 0; e < 4; ++e)
+                if (l + e < n) p |= may(__ldg(r + l + e));
+        }
+        if (lane == 31)  // the four samples past the warp's
+            for (unsigned e = 4; e < 8; ++e)
+                if (l + e < n) p |= may(__ldg(r + l + e));
+        const unsigned any = __ballot_sync(0xffffffffu, p);
+        if (((any >> lane) & 3u) == 0u) continue;
+        for (unsigned e = 0; e < 4; ++e) {
+            const unsigned i = l + e;
+            if (i >= nl) break;
+            const float m = median5(__ldg(r + i), __ldg(r + i + 1), __ldg(r + i + 2),
+                                    __ldg(r + i + 3), __ldg(r + i + 4));
+            if (__fsub_rn(m, mean) >= lim) {
+                const unsigned long long at = atomicAdd(count, 1ull);
+                if ((long long)at < cap) cands[at] = DevCand{row, (int32_t)i, 1, __fdiv_rn(m, rms)};
+            }
         }
     }
 }
@@ -200,8 +554,9 @@ mdsm_status ref_detect_threads(const float *d_series, int ndms, int nsamp, long 
     unsigned nchunks = 1;
     while ((unsigned long long)(nchunks + 1) * mod < vals) ++nchunks;
     if (cap < 0) cap = 0;
-    const size_t off_cnt = 0, off_stats = 16, off_sums = 64;
-    const size_t off_c = off_sums + ((size_t)nchunks * sizeof(double2) + 255) / 256 * 256;
+    const size_t off_cnt = 0, off_stats = 16, off_redo = 32, off_sums = 64;
+    const size_t off_eps = off_sums + ((size_t)nchunks * sizeof(RefChunk) + 255) / 256 * 256;
+    const size_t off_c = off_eps + ((size_t)nchunks * sizeof(float) + 255) / 256 * 256;
     const size_t bytes = off_c + (size_t)std::max<long long>(cap, 1) * sizeof(DevCand);
     void *sc = nullptr;
     std::unique_lock<std::mutex> lease;
@@ -209,12 +564,12 @@ mdsm_status ref_detect_threads(const float *d_series, int ndms, int nsamp, long 
     char *base = static_cast<char *>(sc);
     auto *d_count = reinterpret_cast<unsigned long long *>(base + off_cnt);
     auto *d_stats = reinterpret_cast<float *>(base + off_stats);
-    auto *d_sums = reinterpret_cast<double2 *>(base + off_sums);
     auto *d_c = reinterpret_cast<DevCand *>(base + off_c);
     MDSM_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st));
-    k_ref_chunk_sums<<<(nchunks + 127) / 128, 128, 0, st>>>(d_series, mod, nchunks, d_sums);
-    k_ref_finish<<<1, 1, 0, st>>>(d_sums, mod, nchunks, d_stats);
-    dim3 grid((unsigned)std::min<long long>((nsamp + 255) / 256, 64), (unsigned)ndms);
+    MDSM_TRY(ref_stats(d_series, mod, nchunks, reinterpret_cast<RefChunk *>(base + off_sums),
+                       reinterpret_cast<float *>(base + off_eps),
+                       reinterpret_cast<unsigned *>(base + off_redo), d_stats, st));
+    dim3 grid((unsigned)std::min<long long>((nsamp + 1023) / 1024, 64), (unsigned)ndms);
     k_ref_detect<<<grid, 256, 0, st>>>(d_series, ndms, nsamp, lowdm, dmstep, threshold, d_stats,
                                        d_c, d_count, cap, rpt, tshift);
     MDSM_CUDA_TRY(cudaGetLastError());
@@ -412,7 +767,7 @@ static_assert((unsigned long long)kNoAllocChunks * 32768ull >= 0xFFFFFFFFull / 2
 constexpr long long kNoAllocCands = 65536;
 constexpr size_t kNoAllocHeader = 256;  // counter at 0, statistics at 16
 constexpr size_t kNoAllocBytes =
-    kNoAllocHeader + (size_t)kNoAllocChunks * sizeof(double2) + (size_t)kNoAllocCands * 16;
+    kNoAllocHeader + (size_t)kNoAllocChunks * sizeof(RefChunk) + (size_t)kNoAllocCands * 16;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -450,13 +805,16 @@ mdsm_status ref_detect_noalloc(const float *d_series, int ndms, int nsamp, float
     MDSM_TRY(noalloc_scratch(&base));
     auto *d_count = reinterpret_cast<unsigned long long *>(base);
     auto *d_stats = reinterpret_cast<float *>(base + 16);
-    auto *d_sums = reinterpret_cast<double2 *>(base + kNoAllocHeader);
     auto *d_c = reinterpret_cast<DevCand *>(base + kNoAllocHeader +
-                                            (size_t)kNoAllocChunks * sizeof(double2));
+                                            (size_t)kNoAllocChunks * sizeof(RefChunk));
     MDSM_CUDA_TRY(cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st));
-    k_ref_chunk_sums<<<(nchunks + 127) / 128, 128, 0, st>>>(d_series, mod, nchunks, d_sums);
-    k_ref_finish<<<1, 1, 0, st>>>(d_sums, mod, nchunks, d_stats);
-    dim3 grid((unsigned)std::min<long long>((nsamp + 255) / 256, 64), (unsigned)ndms);
+    // (the chunks' error bounds lie where the candidates go afterwards)
+    static_assert((size_t)kNoAllocChunks * sizeof(float) <= (size_t)kNoAllocCands * sizeof(DevCand),
+                  "the error bounds fit the candidates' place");
+    MDSM_TRY(ref_stats(d_series, mod, nchunks, reinterpret_cast<RefChunk *>(base + kNoAllocHeader),
+                       reinterpret_cast<float *>(d_c), reinterpret_cast<unsigned *>(base + 32),
+                       d_stats, st));
+    dim3 grid((unsigned)std::min<long long>((nsamp + 1023) / 1024, 64), (unsigned)ndms);
     k_ref_detect<<<grid, 256, 0, st>>>(d_series, ndms, nsamp, lowdm, dmstep, threshold, d_stats,
                                        d_c, d_count, cap, ndms, 0);
     MDSM_CUDA_TRY(cudaGetLastError());
