@@ -210,19 +210,31 @@ CAND_DTYPE = np.dtype([("dm_idx", np.int32), ("sample", np.int32), ("snr", np.fl
                        ("width", np.int32)])
 
 
+_CAND_P = ctypes.POINTER(Candidate)
+
+
+def _cand_buffer(cap):
+    """Room for cap candidates (untouched memory: zeroing 16 MB takes longer than most searches)
+    and its pointer."""
+    if cap < 0:
+        raise ValueError("candidate capacity must not be negative")
+    buf = np.empty(max(cap, 1), CAND_DTYPE)
+    return buf, buf.ctypes.data_as(_CAND_P)
+
+
 def _cands_to_array(buf, n):
-    return np.frombuffer(buf, dtype=CAND_DTYPE, count=n).copy()
+    return buf[:n].copy()
 
 
 def ref_detect_device(series, lowdm, dmstep, threshold, cap=1 << 20, stream=None):
     """Reference detector on a device float series [ndms][nsamp].  Returns (cands, mean, rms)
     with cands a structured array sorted by (dm_idx, sample)."""
     ndms, nsamp = series.shape
-    buf = (Candidate * cap)()
+    buf, pbuf = _cand_buffer(cap)
     n = ctypes.c_longlong()
     mean, rms = ctypes.c_float(), ctypes.c_float()
     check(load().mdsm_ref_detect_device(ctypes.c_void_p(series.data_ptr()), ndms, nsamp,
-                                        float(lowdm), float(dmstep), float(threshold), buf, cap,
+                                        float(lowdm), float(dmstep), float(threshold), pbuf, cap,
                                         ctypes.byref(n), ctypes.byref(mean), ctypes.byref(rms),
                                         _stream_ptr(stream)))
     return _cands_to_array(buf, min(n.value, cap)), mean.value, rms.value, n.value
@@ -235,12 +247,12 @@ def ref_detect_chunked_device(series, lowdm, dmstep, threshold, mean, rms, spc, 
     ndms, nsamp = series.shape
     mean = np.ascontiguousarray(mean, np.float32)
     rms = np.ascontiguousarray(rms, np.float32)
-    buf = (Candidate * cap)()
+    buf, pbuf = _cand_buffer(cap)
     n = ctypes.c_longlong()
     check(load().mdsm_ref_detect_chunked_device(
         ctypes.c_void_p(series.data_ptr()), ndms, nsamp, float(lowdm), float(dmstep),
         float(threshold), mean.ctypes.data_as(ctypes.c_void_p),
-        rms.ctypes.data_as(ctypes.c_void_p), mean.size, int(spc), buf, cap, ctypes.byref(n),
+        rms.ctypes.data_as(ctypes.c_void_p), mean.size, int(spc), pbuf, cap, ctypes.byref(n),
         _stream_ptr(stream)))
     return _cands_to_array(buf, min(n.value, cap)), n.value
 
@@ -259,11 +271,11 @@ def ref_detect_subband_device(plan, series, threshold, mean=None, rms=None, spc=
         mp = mean.ctypes.data_as(ctypes.c_void_p)
         rp = rms.ctypes.data_as(ctypes.c_void_p)
         nch = mean.size
-    buf = (Candidate * cap)()
+    buf, pbuf = _cand_buffer(cap)
     n = ctypes.c_longlong()
     check(load().mdsm_ref_detect_subband_device(
         plan._h, ctypes.c_void_p(series.data_ptr()), out_stride, float(threshold), mp, rp, nch,
-        int(spc), buf, cap, ctypes.byref(n), _stream_ptr(stream)))
+        int(spc), pbuf, cap, ctypes.byref(n), _stream_ptr(stream)))
     return _cands_to_array(buf, min(n.value, cap)), n.value
 
 
@@ -272,10 +284,10 @@ def boxcar_detect_device(series, nwidths=9, threshold=6.0, cap=1 << 20, stream=N
     import torch
     ndms, nsamp = series.shape
     dt = 1 if series.dtype == torch.int32 else 0
-    buf = (Candidate * cap)()
+    buf, pbuf = _cand_buffer(cap)
     n = ctypes.c_longlong()
     check(load().mdsm_boxcar_detect_device(ctypes.c_void_p(series.data_ptr()), dt, ndms, nsamp,
-                                           int(nwidths), float(threshold), buf, cap,
+                                           int(nwidths), float(threshold), pbuf, cap,
                                            ctypes.byref(n), _stream_ptr(stream)))
     return _cands_to_array(buf, min(n.value, cap)), n.value
 
@@ -287,11 +299,11 @@ def singlepulse_detect_device(series, max_downfact=30, chunk_len=8000, threshold
     import torch
     ndms, nsamp = series.shape
     dt = 1 if series.dtype == torch.int32 else 0
-    buf = (Candidate * max(cap, 1))()
+    buf, pbuf = _cand_buffer(max(cap, 0))
     n = ctypes.c_longlong()
     check(load().mdsm_singlepulse_detect_device(ctypes.c_void_p(series.data_ptr()), dt, ndms,
                                                 nsamp, int(max_downfact), int(chunk_len),
-                                                int(bool(normalise)), float(threshold), buf, cap,
+                                                int(bool(normalise)), float(threshold), pbuf, cap,
                                                 ctypes.byref(n), _stream_ptr(stream)))
     return _cands_to_array(buf, min(n.value, cap)), n.value
 
