@@ -126,12 +126,8 @@ mdsm_status fused_build(mdsm_batch *b, int shape, int order, bool clip, bool det
         g.d_rel = nullptr;
         g.d_sminspan = nullptr;
         z.geoms[i] = g;
-        // A beam whose staging does not fit this shape (or whose last tile would read past the
-        // caller's buffer, which holds what the plan's own tile shape reads: mdsm_plan_info
-        // in_bytes) runs on its own launches instead.
-        if (fused_tables(shape, z.geoms[i], p.S) != MDSM_OK ||
-            stage_in_bytes(z.geoms[i], b->in_stride[i], 0) >
-                stage_in_bytes(p.stages[0], b->in_stride[i], 0)) {
+        // a beam whose staging does not fit this shape runs on its own launches instead
+        if (fused_tables(shape, z.geoms[i], p.S) != MDSM_OK) {
             free_stage(z.geoms[i]);
             z.rest.push_back((int)i);
             continue;

@@ -245,6 +245,10 @@ struct PackedCfg {
 };
 using CfgU8 = PackedCfg<1, 19, 2>;
 using CfgU8w16 = PackedCfg<1, 16, 2>;         // 32-trial blocks, for trial counts of 32 k
+// 16-trial blocks: half the span of shifts, for plans whose wider blocks do not fit shared memory
+// (they would run one load an add on the generic kernel), and for few trials.
+template <int PT>
+using CfgU8n16 = PackedCfg<1, 16, 1, false, PT>;
 // The first subband stage (uint16 subband series): without the int32 flush registers there
 // is room for 1024-sample tiles, which halve the per-chunk costs per add; 768- or 512-sample
 // tiles where the wider staging does not fit in shared memory.
@@ -282,8 +286,12 @@ __device__ __forceinline__ bool cta_any(bool pred)
     return r != 0;
 }
 
-// Items of one plan, (DM block fastest, time tile, group); CTA b takes b, b + G, b + 2G, ...
+// Items of one plan, (DM block fastest, time tile, part, group); CTA b takes b,
+// b + G, b + 2G, ...  kParts: the channels are cut into a->nsplit parts that add to the output, and
+// the item's first entry is its part.
+template <bool PARTS>
 struct OnePlanItems {
+    static constexpr bool kParts = PARTS;
     const KArgs *a;
     int ntiles, nitems;
     int next_it;
@@ -295,8 +303,18 @@ struct OnePlanItems {
     }
     __device__ int4 item(int it) const
     {
-        const int blk = it % a->nblk, rest = it / a->nblk;
-        return make_int4(0, blk, rest % ntiles, rest / ntiles);
+        const int blk = it % a->nblk, rest = it / a->nblk, part = rest / ntiles;
+        if constexpr (PARTS)
+            return make_int4(part % a->nsplit, blk, rest % ntiles, part / a->nsplit);
+        else
+            return make_int4(0, blk, rest % ntiles, part);
+    }
+    // chunks [x, y) of nch are the item's
+    __device__ int2 chunks(const int4 &w, int nch) const
+    {
+        if constexpr (!PARTS) return make_int2(0, nch);
+        const int per = (nch + a->nsplit - 1) / a->nsplit;
+        return make_int2(w.x * per, min(nch, (w.x + 1) * per));
     }
     __device__ const KArgs &args(int) const { return *a; }
     __device__ void item_done(int) const {}
@@ -315,6 +333,8 @@ struct ListItems {
         return it < nitems ? it : -1;
     }
     __device__ int4 item(int it) const { return items[it]; }
+    __device__ int2 chunks(const int4 &, int nch) const { return make_int2(0, nch); }
+    static constexpr bool kParts = false;
     __device__ const KArgs &args(int beam) const { return beams[beam]; }
     __device__ void item_done(int) const {}
     static constexpr bool kBeamStride = true;  // each beam's chunks with its own phase stride
@@ -361,7 +381,8 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
     if (warp == NW) {
         // ---- producer: the item being staged, its next chunk, and the lane's (smin, span)
         // for that chunk, loaded one fill ahead so that no fill waits on a global load
-        int p_it = -1, p_k = 0, p_nchunks = 0;
+        int p_it = -1, p_k = 0;
+        int2 p_ks = make_int2(0, 0);  // the item's chunks
         int4 p_w = make_int4(0, 0, 0, 0);
         int2 p_ss = make_int2(0, 0);
         // the item's beam fields the fills use, in registers (the barrier and copy asm clobber
@@ -370,13 +391,12 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
             const unsigned char *in;
             long long in_stride, in_group_stride;
             const int32_t *rel, *sminspan;
-            int nchans, nblk;
+            int nchans, nblk, nsamp;
         } a{};
         auto p_next_item = [&]() {
             int it = 0;
             if (lane == 0) it = src.grab();
             p_it = __shfl_sync(0xffffffffu, it, 0);
-            p_k = 0;
             if (p_it >= 0) {
                 p_w = src.item(p_it);
                 const KArgs &b = src.args(p_w.x);
@@ -387,7 +407,9 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
                 a.sminspan = b.sminspan;
                 a.nchans = b.nchans;
                 a.nblk = b.nblk;
-                p_nchunks = (a.nchans + kPCC - 1) / kPCC;
+                a.nsamp = b.nsamp;
+                p_ks = src.chunks(p_w, (a.nchans + kPCC - 1) / kPCC);
+                p_k = p_ks.x;
             }
         };
         auto p_load_ss = [&]() {
@@ -417,7 +439,9 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
             if (lane < nc) {
                 const int c = c0 + lane;
                 const long long start = t0 + p_ss.x;
-                const long long end = start + Cfg::PT + p_ss.y;
+                // (no sample past the last output's is read)
+                const long long end =
+                    start + min((long long)Cfg::PT, (long long)a.nsamp - t0) + p_ss.y;
                 const long long sb = (start * SW) & ~15LL;  // bytes
                 const long long eb = (end * SW + 15) & ~15LL;
                 bytes = (unsigned)(eb - sb);
@@ -429,8 +453,8 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
             __syncwarp();
             if (lane == 0) {
                 meta[s] = make_int4(p_it, p_k, nc,
-                                    (p_k == 0 ? kChunkFirst : 0) |
-                                        (p_k == p_nchunks - 1 ? kChunkLast : 0) |
+                                    (p_k == p_ks.x ? kChunkFirst : 0) |
+                                        (p_k == p_ks.y - 1 ? kChunkLast : 0) |
                                         (p_w.x << 8));  // the item's beam above the flags
                 mbar_arrive_expect_tx(&bars[s], total);  // releases the meta entry with the phase
             }
@@ -440,7 +464,7 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
             if (lane == 0)
                 bulk_g2s(offsm + s * kPCC * DBS, a.rel + (bofs + (size_t)c0) * DBS, offbytes,
                          &bars[s]);
-            if (++p_k == p_nchunks) p_next_item();
+            if (++p_k == p_ks.y) p_next_item();
             p_load_ss();
         };
         // One CTA barrier per chunk, as the compute warps', then the refill of the stage every
@@ -647,6 +671,11 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
         const long long t0 = (long long)w.z * Cfg::PT;
         constexpr bool U16OUT = Cfg::U16OUT;
         constexpr int osz = U16OUT ? 2 : 4;
+        uint32_t nadded = (uint32_t)a.nchans;  // the item's channels
+        if constexpr (Src::kParts) {
+            const int2 ks = src.chunks(w, (a.nchans + kPCC - 1) / kPCC);
+            nadded = (uint32_t)(min(a.nchans, ks.y * kPCC) - ks.x * kPCC);
+        }
 #pragma unroll
         for (int j = 0; j < DPW; ++j) {
             const int d = w.y * DB + warp * DPW + j;
@@ -679,7 +708,7 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
                 if constexpr (SW == 2) {
                     // offset-binary sums less 32768 per channel (exact: the host keeps
                     // nchans * 65535 below 2^31)
-                    const uint32_t bias = Cfg::SIGNED ? 32768u * (uint32_t)a.nchans : 0u;
+                    const uint32_t bias = Cfg::SIGNED ? 32768u * nadded : 0u;
                     v[0] = (int32_t)(A[j][r] - (O[j][r] << 16) - bias);
                     v[SPW - 1] = (int32_t)(O[j][r] - bias);
                 } else {
@@ -696,6 +725,17 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
                             m2lo += q;
                             m2hi += (m2lo < q);
                         }
+                }
+                if constexpr (Src::kParts) {  // a part of the channels adds its sums
+#pragma unroll
+                    for (int e = 0; e < SPW; ++e)
+                        if (t + e < a.nsamp) {
+                            if (a.out_i32)
+                                atomicAdd(reinterpret_cast<int *>(orow) + t + e, v[e]);
+                            else  // (whole numbers below 2^24: exact in any order)
+                                atomicAdd(reinterpret_cast<float *>(orow) + t + e, (float)v[e]);
+                        }
+                    continue;
                 }
                 if (whole && a.out_i32) {
                     if constexpr (SPW == 4)
@@ -755,13 +795,13 @@ __device__ __forceinline__ void packed_init_barriers(unsigned char *smem)
 }
 
 // One plan: a persistent grid of at most one CTA per SM over the plan's items.
-template <class Cfg>
+template <class Cfg, bool PARTS = false>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
     k_shift_sum_packed(const __grid_constant__ KArgs a, int ntiles, int nitems)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     packed_init_barriers(smem);
-    OnePlanItems src{&a, ntiles, nitems, (int)blockIdx.x};
+    OnePlanItems<PARTS> src{&a, ntiles, nitems, (int)blockIdx.x};
     packed_stream<Cfg>(src, smem, a.rowcap, a.ps, a.err);
 }
 
@@ -856,6 +896,8 @@ struct FusedItems {
         return it;
     }
     __device__ int4 item(int it) const { return items[it]; }
+    __device__ int2 chunks(const int4 &, int nch) const { return make_int2(0, nch); }
+    static constexpr bool kParts = false;
     __device__ const KArgs &args(int beam) const { return beams[beam]; }
     __device__ void item_done(int beam) const
     {
@@ -1110,6 +1152,26 @@ int tile_tables(StageGeom &g, const std::vector<int32_t> &S)
     return maxspan;
 }
 
+// Bytes of a phase copy of a staged row (packed_tables' ps) for blocks of db trials, from the
+// spans of the first and the last channel (delays grow along the band, so one of them has the
+// widest; packed_tables looks at every channel).
+int packed_row(const StageGeom &g, const std::vector<int32_t> &S, int db, int pt, int sw)
+{
+    int maxspan = 0;
+    for (int c : {0, g.nchans - 1})
+        for (int gi = 0; gi < g.ngroups; ++gi)
+            for (int d0 = 0; d0 < g.ndms; d0 += db) {
+                int lo = INT32_MAX, hi = INT32_MIN;
+                for (int d = d0; d < std::min(g.ndms, d0 + db); ++d) {
+                    const int v = S[((size_t)gi * g.ndms + d) * g.nchans + c];
+                    lo = std::min(lo, v);
+                    hi = std::max(hi, v);
+                }
+                maxspan = std::max(maxspan, hi - lo);
+            }
+    return (int)(((long long)(pt + maxspan) * sw + 32 + 15) / 16 * 16);
+}
+
 // Dynamic shared memory a packed CTA may take: the device's opt-in limit per block (227 KB on
 // GB300; the packed kernels declare no static shared memory), 220 KB if it cannot be read.
 size_t packed_smem_limit()
@@ -1171,6 +1233,91 @@ bool packed_tables(StageGeom &g, const std::vector<int32_t> &S, int kernel_id)
     g.smem_bytes = packed_smem<Cfg>(rawcap, ps);
     g.kernel = kernel_id;
     return true;
+}
+
+}  // namespace
+
+// The uint8 tile shapes; packed_clocks orders those that fit.
+namespace {
+
+struct PackedShape {
+    int sw, db, pt, threads;
+    double per_wave;  // clocks of a chunk per shared-memory wavefront, measured
+    bool (*tables)(StageGeom &, const std::vector<int32_t> &, int);
+    size_t (*smem)(int rawcap, int ps);
+    const void *fn, *fn_parts;
+};
+template <class Cfg>
+PackedShape packed_shape(double per_wave)
+{
+    return {Cfg::SW, Cfg::DB, Cfg::PT, Cfg::THREADS, per_wave, &packed_tables<Cfg>, &packed_smem<Cfg>,
+            reinterpret_cast<const void *>(&k_shift_sum_packed<Cfg>),
+            reinterpret_cast<const void *>(&k_shift_sum_packed<Cfg, true>)};
+}
+const PackedShape kU8Shapes[] = {packed_shape<CfgU8>(1.32), packed_shape<CfgU8w16>(1.45),
+                                 packed_shape<CfgU8n16<768>>(1.58), packed_shape<CfgU8n16<512>>(1.75)};
+constexpr int kNumU8Shapes = 4;
+// 16-bit samples: 768 or 512 samples, unsigned and signed.
+const PackedShape kU16Shapes[] = {packed_shape<CfgU16T<768>>(1.35), packed_shape<CfgU16T<512>>(1.35),
+                                  packed_shape<CfgI16T<768>>(1.35), packed_shape<CfgI16T<512>>(1.35)};
+
+// The shape of a stage that a packed kernel with 32-bit output runs.
+const PackedShape &packed_shape_of(const StageGeom &g)
+{
+    if (g.kernel == 2) return kU8Shapes[g.variant];
+    return kU16Shapes[(g.in_dtype == MDSM_I16 ? 2 : 0) + (g.T == 768 ? 0 : 1)];
+}
+
+int device_sms()
+{
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = 152;
+    }
+    return n;
+}
+
+// Clocks of a launch over `items` tiles with the channels cut into `split` parts, each its own
+// item (row: bytes of a phase copy).  A chunk of 16 channels takes the shared-memory wavefronts of
+// its words, its offsets and its expansion (8 per 512 bytes of a row to read it and 4 to write
+// each phase copy) at the shape's measured rate (more warps and trials a warp hide more latency), and at least
+// 1500 clocks: the 17 bulk copies it is staged by are issued at 70 clocks each.  A part adds its sums to the output with atomics.
+double packed_clocks(const PackedShape &z, int row, int nchans, double items, int split, int sms)
+{
+    const double lsu = 16.0 * z.db * z.pt * z.sw / 128.0 + 16.0 * (z.threads / 32) +
+                       16.0 * row / 512.0 * (8 + 16 / z.sw);
+    const double chunk = std::max(1500.0, z.per_wave * lsu);
+    const int nch = (nchans + 15) / 16, per = (nch + split - 1) / split;
+    return std::ceil(items * split / sms) * (per * chunk + (split > 1 ? 4000.0 : 1500.0)) +
+           (split > 1 ? 6000.0 : 0.0);
+}
+
+// The number of parts with the lowest estimate: one where a call has many tiles for the SMs;
+// more where the last wave of them (or the only one) would leave SMs idle.  No part is empty.
+int packed_split(const PackedShape &z, int row, int nchans, double items, int sms)
+{
+    const int nch = (nchans + 15) / 16;
+    int best = 1;
+    double clk = packed_clocks(z, row, nchans, items, 1, sms);
+    for (int per = std::max(1, nch / 2); per >= 1 && nch / per <= 32; --per) {
+        const int split = (nch + per - 1) / per;
+        const double c = packed_clocks(z, row, nchans, items, split, sms);
+        if (c < 0.95 * clk) {
+            clk = c;
+            best = split;
+        }
+    }
+    return best;
+}
+
+// Whether a packed stage's sums may be added up from parts: one group, and float output only where
+// every partial sum is a whole number within 2^24, exact in float in any order.
+bool packed_may_split(const StageGeom &g)
+{
+    const long long most = g.in_dtype == MDSM_U8 ? 255 : g.in_dtype == MDSM_I16 ? 32768 : 65535;
+    return g.ngroups == 1 && !g.out_u16 && (g.out_i32 || g.nchans * most <= (1 << 24));
 }
 
 }  // namespace
@@ -1298,12 +1445,12 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
     // the packed kernels sum exactly in int32: only where every sum fits
     if (g.kernel != 1) {
         if (g.in_dtype == MDSM_U8 && (long long)g.nchans * 255 <= 0x7fffffffLL) {
-            // 38-trial blocks run ~5 % faster per trial than 32-trial ones; take 32 where the
-            // last 38-trial block would leave more than that idle (e.g. 64 or 128 trials)
-            const int n38 = (g.ndms + CfgU8::DB - 1) / CfgU8::DB * CfgU8::DB;
-            const int n32 = (g.ndms + CfgU8w16::DB - 1) / CfgU8w16::DB * CfgU8w16::DB;
-            const bool w38 = n38 <= 1.05 * n32;
             if (g.out_u16) {
+                // 38-trial blocks run ~5 % faster per trial than 32-trial ones; take 32 where the
+                // last 38-trial block would leave more than that idle (e.g. 64 or 128 trials)
+                const int n38 = (g.ndms + CfgU8::DB - 1) / CfgU8::DB * CfgU8::DB;
+                const int n32 = (g.ndms + CfgU8w16::DB - 1) / CfgU8w16::DB * CfgU8w16::DB;
+                const bool w38 = n38 <= 1.05 * n32;
                 if (w38 && (packed_tables<CfgU8to16T<19, 1024>>(g, S, 2) ||
                             packed_tables<CfgU8to16T<19, 768>>(g, S, 2) ||
                             packed_tables<CfgU8to16T<19, 512>>(g, S, 2)))
@@ -1313,8 +1460,26 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
                     packed_tables<CfgU8to16T<16, 512>>(g, S, 2))
                     return MDSM_OK;
             } else {
-                if (w38 && packed_tables<CfgU8>(g, S, 2)) return MDSM_OK;
-                if (packed_tables<CfgU8w16>(g, S, 2)) return MDSM_OK;
+                // the shape with the lowest estimate: 38 trials x 512 samples where their span of
+                // shifts fits and few of the trials idle (53 % of the add peak), else 32 or 16
+                const int sms = device_sms();
+                std::vector<std::pair<double, int>> order;
+                for (int i = 0; i < kNumU8Shapes; ++i) {
+                    const PackedShape &z = kU8Shapes[i];
+                    const int row = packed_row(g, S, z.db, z.pt, 1);
+                    if (z.smem(row + 16, row) > packed_smem_limit() || row >= 4096) continue;
+                    const double items = (double)((g.ndms + z.db - 1) / z.db) *
+                                         ((g.nsamp + z.pt - 1) / z.pt) * g.ngroups;
+                    const int split =
+                        packed_may_split(g) ? packed_split(z, row, g.nchans, items, sms) : 1;
+                    order.emplace_back(packed_clocks(z, row, g.nchans, items, split, sms), i);
+                }
+                std::sort(order.begin(), order.end());
+                for (const auto &o : order)
+                    if (kU8Shapes[o.second].tables(g, S, 2)) {
+                        g.variant = o.second;
+                        return MDSM_OK;
+                    }
             }
         }
         if ((g.in_dtype == MDSM_U16 || g.in_dtype == MDSM_I16) && !g.out_u16 &&
@@ -1330,6 +1495,11 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
     // Try Db = 32, 16, 8 until the staged rows fit in shared memory.
     const int dpws[3] = {4, 2, 1};
     int first = g.DPW == 4 ? 0 : (g.DPW == 2 ? 1 : 2);
+    // fewer trials a block where the call would otherwise not fill the SMs (two CTAs each)
+    if (g.fill_sms)
+        while (first < 2 && (double)((g.ndms + kNW * dpws[first] - 1) / (kNW * dpws[first])) *
+                                    ((g.nsamp + g.T - 1) / g.T) * g.ngroups < 2.0 * device_sms())
+            ++first;
     for (int i = first; i < 3; ++i) {
         g.DPW = dpws[i];
         g.Db = kNW * g.DPW;
@@ -1378,6 +1548,14 @@ long long stage_in_bytes(const StageGeom &g, long long in_stride, long long in_g
                SZ + last;
 }
 
+long long stage_reads(const StageGeom &g, long long in_stride, long long in_group_stride)
+{
+    if (g.kernel == 1) return stage_in_bytes(g, in_stride, in_group_stride);
+    const long long SZ = (long long)dtype_size(g.in_dtype);
+    return ((long long)(g.ngroups - 1) * in_group_stride + (long long)(g.nchans - 1) * in_stride) *
+               SZ + (((long long)g.nsamp + g.max_shift) * SZ + 15) / 16 * 16;
+}
+
 mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride,
                          long long in_group_stride, void *out, long long out_stride,
                          long long out_group_stride, unsigned *d_err, cudaStream_t st,
@@ -1395,25 +1573,28 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
     void *fn = select_kernel(g.in_dtype, g.acc_int, g.DPW, g.cc);
     unsigned threads = kNW * 32;
     bool persistent = true;  // the packed kernels: a persistent grid over (block, tile, group)
-    if (g.kernel == 2 && g.Db == CfgU8::DB) {
-        fn = !g.out_u16     ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8>)
-             : g.T == 1024 ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<19, 1024>>)
+    const long long ntiles = (nsamp + g.T - 1) / g.T;
+    long long nitems = (long long)g.nblk * ntiles * g.ngroups;
+    const int sms = device_sms();
+    if (!(mom && stage_folds_moments(g))) mom = nullptr;
+    int nsplit = 1;
+    if (g.kernel == 3 || (g.kernel == 2 && !g.out_u16)) {
+        const PackedShape &z = packed_shape_of(g);
+        if (!mom && packed_may_split(g))
+            nsplit = packed_split(z, g.ps, g.nchans, (double)nitems, sms);
+        nitems *= nsplit;
+        fn = const_cast<void *>(nsplit > 1 ? z.fn_parts : z.fn);
+        threads = (unsigned)z.threads;
+    } else if (g.kernel == 2 && g.Db == CfgU8::DB) {
+        fn = g.T == 1024 ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<19, 1024>>)
              : g.T == 768  ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<19, 768>>)
                            : reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<19, 512>>);
         threads = CfgU8::THREADS;
     } else if (g.kernel == 2) {
-        fn = !g.out_u16     ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8w16>)
-             : g.T == 1024 ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<16, 1024>>)
+        fn = g.T == 1024 ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<16, 1024>>)
              : g.T == 768  ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<16, 768>>)
                            : reinterpret_cast<void *>(&k_shift_sum_packed<CfgU8to16T<16, 512>>);
         threads = CfgU8w16::THREADS;
-    } else if (g.kernel == 3) {
-        const bool sgn = g.in_dtype == MDSM_I16;
-        fn = g.T == 768 ? (sgn ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgI16T<768>>)
-                               : reinterpret_cast<void *>(&k_shift_sum_packed<CfgU16T<768>>))
-                        : (sgn ? reinterpret_cast<void *>(&k_shift_sum_packed<CfgI16T<512>>)
-                               : reinterpret_cast<void *>(&k_shift_sum_packed<CfgU16T<512>>));
-        threads = CfgU16T<512>::THREADS;
     } else {
         persistent = false;
     }
@@ -1437,16 +1618,15 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
     a.out_i32 = g.out_i32;
     a.ps = g.ps;
     a.err = d_err;
-    a.mom = (mom && stage_folds_moments(g)) ? mom : nullptr;
+    a.mom = mom;
     a.mom_group_rows = mom_group_rows;
-    const long long ntiles = (nsamp + g.T - 1) / g.T;
+    a.nsplit = nsplit;
     if (persistent) {
-        // at most one CTA per SM walks the (DM block, tile, group) items
-        const long long nitems = (long long)g.nblk * ntiles * g.ngroups;
+        // a persistent grid walks the (DM block, tile, group) items
+        if (nsplit > 1)  // the parts add to zeros
+            MDSM_CUDA_TRY(cudaMemset2DAsync(out, (size_t)out_stride * 4, 0, (size_t)nsamp * 4,
+                                            (size_t)g.ndms, st));
         if (nitems > 0x7fffffffLL) return fail(MDSM_EINVAL, "block too long for one launch");
-        int dev = 0, sms = 0;
-        MDSM_CUDA_TRY(cudaGetDevice(&dev));
-        MDSM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         int nt = (int)ntiles, ni = (int)nitems;
         void *args[] = {&a, &nt, &ni};
         const unsigned grid = (unsigned)std::min<long long>(sms, nitems);

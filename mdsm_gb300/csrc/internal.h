@@ -60,6 +60,7 @@ struct KArgs {
     const int32_t *sminspan;                 // [g][blk][c][2]
     int nchans, ndms, nsamp, nblk, rowcap, nst, out_i32;
     int ps;  // packed kernels: bytes per phase copy of a staged row
+    int nsplit;  // one-plan packed launches: parts of the channels, each added to the output
     unsigned *err;
     // optional (packed kernels, int32 output): exact moments of every output row, accumulated
     // as the row is stored -- (sum, sum of squares low 64 bits, high 64 bits) per row at
@@ -98,6 +99,8 @@ struct StageGeom {
     int ps = 0;           // packed kernels: bytes per phase copy of a staged row
     int kernel = 0;       // requested (0 choose, 1 generic); after tiling: 1 generic, 2 packed
                           // uint8, 3 packed uint16
+    bool fill_sms = true; // the generic kernel's block may shrink to fill the SMs
+    int variant = 0;      // packed uint8 kernel (not uint16 output): its tile shape
 };
 
 // Build the blocked tables of a stage from a full shift table S[g][d][c] (row-major).  Picks
@@ -108,6 +111,8 @@ mdsm_status upload_stage(StageGeom &g);
 void free_stage(StageGeom &g);
 // Bytes of input (from the group base) the kernel may read for in_stride, with tile overrun.
 long long stage_in_bytes(const StageGeom &g, long long in_stride, long long in_group_stride);
+// Bytes it does read: the packed kernels stop at the last output's last sample.
+long long stage_reads(const StageGeom &g, long long in_stride, long long in_group_stride);
 // Launch the stage kernel.  Returns number of kernels launched via *launches.
 // nsamp_run >= 0 computes only output samples [0, nsamp_run) (a time segment of the block,
 // with in/out already offset to its first sample); -1 computes all g.nsamp.

@@ -184,6 +184,7 @@ mdsm_status plan_create_brute(const mdsm_brute_desc &d, Plan &p)
     g.out_i32 = d.out_dtype == MDSM_OUT_I32;
     g.DPW = d.dm_block == 16 ? 2 : (d.dm_block == 8 ? 1 : 4);
     g.kernel = d.kernel;
+    g.fill_sms = d.dm_block == 0;
     MDSM_TRY(build_stage_tables(g, p.S));
     p.maxshift = g.max_shift;
     MDSM_TRY(upload_stage(g));
@@ -404,19 +405,20 @@ mdsm_status plan_create_subband(const mdsm_subband_desc &d, Plan &p)
 // running a plan
 // --------------------------------------------------------------------------------------------
 
-mdsm_status plan_in_requirements(const Plan &p, long long in_stride, long long *in_bytes)
+static mdsm_status plan_reads(const Plan &p, long long in_stride, long long *in_bytes,
+                              long long (*stage)(const StageGeom &, long long, long long))
 {
     if (in_stride < (long long)p.nsamp + p.maxshift)
         return fail(MDSM_ERANGE, "input row pitch smaller than nsamp + maxshift (" +
                                      std::to_string(p.nsamp + p.maxshift) + ")");
     long long need = 0;
     if (p.kind == 1) {
-        need = stage_in_bytes(p.stages[0], in_stride, 0);
+        need = stage(p.stages[0], in_stride, 0);
     } else {
         for (size_t i = 0; i < p.stages.size(); i += 2) {
             const StageGeom &g1 = p.stages[i];
             if (p.pass_bin[i / 2] == 1)
-                need = std::max(need, stage_in_bytes(g1, in_stride, g1.in_group_stride * in_stride));
+                need = std::max(need, stage(g1, in_stride, g1.in_group_stride * in_stride));
             else  // the downsampling kernel reads whole rows of nsamp + maxshift samples
                 need = std::max(need, ((long long)(p.nchans - 1) * in_stride + p.nsamp +
                                        p.maxshift) * (long long)dtype_size(p.in_dtype));
@@ -426,12 +428,17 @@ mdsm_status plan_in_requirements(const Plan &p, long long in_stride, long long *
     return MDSM_OK;
 }
 
+mdsm_status plan_in_requirements(const Plan &p, long long in_stride, long long *in_bytes)
+{
+    return plan_reads(p, in_stride, in_bytes, &stage_in_bytes);
+}
+
 mdsm_status plan_run_device(Plan &p, const void *d_in, long long in_stride, size_t in_bytes,
                             void *d_out, long long out_stride, cudaStream_t st,
                             unsigned long long *mom, bool *folded)
 {
     long long need = 0;
-    MDSM_TRY(plan_in_requirements(p, in_stride, &need));
+    MDSM_TRY(plan_reads(p, in_stride, &need, &stage_reads));
     if ((long long)in_bytes < need)
         return fail(MDSM_ERANGE, "input buffer has " + std::to_string(in_bytes) +
                                      " bytes; the plan reads up to " + std::to_string(need));
