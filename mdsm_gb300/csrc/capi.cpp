@@ -38,7 +38,10 @@ namespace {
 
 void plan_release(Plan &p)
 {
-    for (auto &g : p.stages) free_stage(g);
+    for (auto &g : p.stages) {
+        free_stage(g);
+        tm_release(g.tm);
+    }
     if (p.d_work) cudaFree(p.d_work);
     if (p.d_ds) cudaFree(p.d_ds);
     p.d_ds = nullptr;
@@ -218,9 +221,13 @@ mdsm_status mdsm_plan_get_info(const mdsm_plan *plan, mdsm_plan_info *info)
     info->in_dtype = p.in_dtype;
     info->out_dtype = p.out_dtype;
     info->acc = p.acc;
-    info->dm_block = p.stages.empty() ? 0 : p.stages.back().Db;
-    info->time_tile = p.stages.empty() ? 0 : p.stages.back().T;
-    info->kernel = p.stages.empty() ? 0 : p.stages.back().kernel;
+    if (!p.stages.empty()) {
+        const StageGeom &g = p.stages.back();
+        const bool tm = g.tm.shape >= 0;
+        info->dm_block = tm ? g.tm.DB : g.Db;
+        info->time_tile = tm ? g.tm.T : g.T;
+        info->kernel = tm ? 4 : g.kernel;
+    }
     info->nstages = (int)p.stages.size();
     info->work_bytes = (long long)p.work_bytes;
     return MDSM_OK;
@@ -233,15 +240,16 @@ mdsm_status mdsm_plan_stage_info(const mdsm_plan *plan, int stage, mdsm_stage_in
     if (stage < 0 || stage >= (int)p.stages.size()) return fail(MDSM_EINVAL, "no such stage");
     const StageGeom &g = p.stages[(size_t)stage];
     std::memset(info, 0, sizeof(*info));
-    info->kernel = g.kernel;
-    info->dm_block = g.Db;
-    info->time_tile = g.T;
+    const bool tm = g.tm.shape >= 0;
+    info->kernel = tm ? 4 : g.kernel;
+    info->dm_block = tm ? g.tm.DB : g.Db;
+    info->time_tile = tm ? g.tm.T : g.T;
     info->out_u16 = g.out_u16;
     info->nchans = g.nchans;
     info->ndms = g.ndms;
     info->ngroups = g.ngroups;
     info->nsamp = (int)g.nsamp;
-    info->smem_bytes = (long long)g.smem_bytes;
+    info->smem_bytes = (long long)(tm ? g.tm.smem : g.smem_bytes);
     return MDSM_OK;
 }
 

@@ -1122,6 +1122,17 @@ size_t dtype_size(int dtype)
     }
 }
 
+int device_sms()
+{
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        n = 152;
+    }
+    return n;
+}
+
 namespace {
 
 // Per-block (smin, span) and relative shifts of S[g][d][c] for DM blocks of g.Db.
@@ -1266,17 +1277,6 @@ const PackedShape &packed_shape_of(const StageGeom &g)
 {
     if (g.kernel == 2) return kU8Shapes[g.variant];
     return kU16Shapes[(g.in_dtype == MDSM_I16 ? 2 : 0) + (g.T == 768 ? 0 : 1)];
-}
-
-int device_sms()
-{
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-        cudaGetLastError();
-        n = 152;
-    }
-    return n;
 }
 
 // Clocks of a launch over `items` tiles with the channels cut into `split` parts, each its own
@@ -1570,6 +1570,12 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
         return fail(MDSM_EINVAL, "input row pitch must be a multiple of 16 bytes");
     if ((in_group_stride * SZ) % 16 != 0)
         return fail(MDSM_EINVAL, "input group pitch must be a multiple of 16 bytes");
+    if (g.tm.shape >= 0) {
+        MDSM_TRY(tm_launch(g, in, in_stride, in_group_stride, out, out_stride, out_group_stride,
+                           d_err, st, nsamp));
+        if (launches) *launches += 1;
+        return MDSM_OK;
+    }
     void *fn = select_kernel(g.in_dtype, g.acc_int, g.DPW, g.cc);
     unsigned threads = kNW * 32;
     bool persistent = true;  // the packed kernels: a persistent grid over (block, tile, group)

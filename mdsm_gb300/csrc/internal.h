@@ -72,6 +72,23 @@ struct KArgs {
 // ----------------------------------------------------------------------------------------
 // one launch of the generic shift-and-sum kernel: out[g][d][t] = sum_c in[g][c][t + S[g][d][c]]
 // ----------------------------------------------------------------------------------------
+// tables of a stage's tensor-memory form (tmsum.cu); shape -1: the stage has none
+struct TmStage {
+    int shape = -1;            // index of its kernel
+    int nblk = 0, DB = 0, T = 0;
+    int ncmax = 0;             // channels of the largest chunk
+    int nst = 0;               // chunks in the shared-memory ring
+    int rowcap = 0;            // bytes of a staged row
+    size_t smem = 0, noff = 0;
+    // host tables, until they are uploaded
+    std::vector<uint16_t> offs;
+    std::vector<int4> chunks;
+    std::vector<int> chunk0;
+    std::vector<int2> chan;
+    void *d_tab = nullptr;     // offsets, then chunks, chunk0 and chan at these bytes
+    size_t o_chunks = 0, o_chunk0 = 0, o_chan = 0;
+};
+
 struct StageGeom {
     int nchans = 0;   // channels summed per group
     int ndms = 0;     // output rows per group
@@ -101,7 +118,21 @@ struct StageGeom {
                           // uint8, 3 packed uint16
     bool fill_sms = true; // the generic kernel's block may shrink to fill the SMs
     int variant = 0;      // packed uint8 kernel (not uint16 output): its tile shape
+    bool no_tm = false;   // never the tensor-memory form (the generic kernel asked for)
+    TmStage tm;           // where present it runs the stage; Db, T, kernel and the tables above
+                          // are those of the shared-memory kernels (batched launches, buffers)
 };
+
+// The tensor-memory form of a stage of float samples (tmsum.cu): its tables from the full shift table,
+// where one of its shapes fits and is estimated faster; their upload; the launch.
+int device_sms();
+mdsm_status tm_build(StageGeom &g, const std::vector<int32_t> &S);
+mdsm_status tm_upload(TmStage &t);
+void tm_release(TmStage &t);
+mdsm_status tm_launch(const StageGeom &g, const void *in, long long in_stride,
+                      long long in_group_stride, void *out, long long out_stride,
+                      long long out_group_stride, unsigned *d_err, cudaStream_t st,
+                      long long nsamp);
 
 // Build the blocked tables of a stage from a full shift table S[g][d][c] (row-major).  Picks
 // the tile shape: Db starts at 8*DPW (DPW as set on entry) and shrinks until the staged rows

@@ -185,9 +185,12 @@ mdsm_status plan_create_brute(const mdsm_brute_desc &d, Plan &p)
     g.DPW = d.dm_block == 16 ? 2 : (d.dm_block == 8 ? 1 : 4);
     g.kernel = d.kernel;
     g.fill_sms = d.dm_block == 0;
+    g.no_tm = d.kernel == 1 || d.dm_block != 0;
     MDSM_TRY(build_stage_tables(g, p.S));
+    MDSM_TRY(tm_build(g, p.S));
     p.maxshift = g.max_shift;
     MDSM_TRY(upload_stage(g));
+    MDSM_TRY(tm_upload(g.tm));
     p.stages.push_back(std::move(g));
     p.in_stride = round_pitch((long long)p.nsamp + p.maxshift, p.in_dtype);
     return alloc_err(p);
@@ -332,6 +335,7 @@ mdsm_status plan_create_subband(const mdsm_subband_desc &d, Plan &p)
                 for (int c = 0; c < cps; ++c)
                     S1g[((size_t)b * ncalls + j) * cps + c] = S1[(size_t)j * d.nchans + b * cps + c];
         MDSM_TRY(build_stage_tables(g1, S1g));
+        MDSM_TRY(tm_build(g1, S1g));
         const int pz = g1.out_u16 ? MDSM_U16 : zdtype;  // the pass's subband series type
         const long long n1p = round_pitch(n1, pz);
         m1 = g1.max_shift;
@@ -349,11 +353,14 @@ mdsm_status plan_create_subband(const mdsm_subband_desc &d, Plan &p)
         g2.DPW = calldms <= 8 ? 1 : (calldms <= 16 ? 2 : 4);  // DM block no wider than a call
         if (calldms < 10) g2.kernel = 1;  // the packed uint16 kernel's blocks are 16 trials
         MDSM_TRY(build_stage_tables(g2, S2));
+        MDSM_TRY(tm_build(g2, S2));
         g2.in_stride = n1p;
         g2.in_group_stride = (long long)nsubs * n1p;
         g1.in_group_stride = cps;  // multiplied by the input pitch at run time
         MDSM_TRY(upload_stage(g1));
         MDSM_TRY(upload_stage(g2));
+        MDSM_TRY(tm_upload(g1.tm));
+        MDSM_TRY(tm_upload(g2.tm));
         // z is written for t < n1 and read with the stage-2 tile overrun past its last row
         const size_t zwrite = (size_t)ncalls * nsubs * n1p * dtype_size(pz);
         const size_t zread = (size_t)stage_in_bytes(g2, n1p, (long long)nsubs * n1p);
