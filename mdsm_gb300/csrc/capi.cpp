@@ -41,6 +41,7 @@ void plan_release(Plan &p)
     for (auto &g : p.stages) {
         free_stage(g);
         tm_release(g.tm);
+        gs_release(g.gs);
     }
     if (p.d_work) cudaFree(p.d_work);
     if (p.d_ds) cudaFree(p.d_ds);
@@ -223,9 +224,9 @@ mdsm_status mdsm_plan_get_info(const mdsm_plan *plan, mdsm_plan_info *info)
     info->acc = p.acc;
     if (!p.stages.empty()) {
         const StageGeom &g = p.stages.back();
-        const bool tm = g.tm.shape >= 0;
-        info->dm_block = tm ? g.tm.DB : g.Db;
-        info->time_tile = tm ? g.tm.T : g.T;
+        const bool tm = g.tm.shape >= 0, gs = g.gs.shape >= 0;
+        info->dm_block = tm ? g.tm.DB : gs ? g.gs.DB : g.Db;
+        info->time_tile = tm ? g.tm.T : gs ? g.gs.T : g.T;
         info->kernel = tm ? 4 : g.kernel;
     }
     info->nstages = (int)p.stages.size();
@@ -240,16 +241,16 @@ mdsm_status mdsm_plan_stage_info(const mdsm_plan *plan, int stage, mdsm_stage_in
     if (stage < 0 || stage >= (int)p.stages.size()) return fail(MDSM_EINVAL, "no such stage");
     const StageGeom &g = p.stages[(size_t)stage];
     std::memset(info, 0, sizeof(*info));
-    const bool tm = g.tm.shape >= 0;
+    const bool tm = g.tm.shape >= 0, gs = g.gs.shape >= 0;
     info->kernel = tm ? 4 : g.kernel;
-    info->dm_block = tm ? g.tm.DB : g.Db;
-    info->time_tile = tm ? g.tm.T : g.T;
+    info->dm_block = tm ? g.tm.DB : gs ? g.gs.DB : g.Db;
+    info->time_tile = tm ? g.tm.T : gs ? g.gs.T : g.T;
     info->out_u16 = g.out_u16;
     info->nchans = g.nchans;
     info->ndms = g.ndms;
     info->ngroups = g.ngroups;
     info->nsamp = (int)g.nsamp;
-    info->smem_bytes = (long long)(tm ? g.tm.smem : g.smem_bytes);
+    info->smem_bytes = (long long)(tm ? g.tm.smem : gs ? g.gs.smem : g.smem_bytes);
     return MDSM_OK;
 }
 

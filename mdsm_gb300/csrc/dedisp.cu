@@ -269,23 +269,6 @@ using CfgI16T = PackedCfg<2, 16, 1, false, PT, true>;
 // (few channels, as in the subband stages) keep the copies in flight between items.
 constexpr int kChunkFirst = 1, kChunkLast = 2, kChunkStop = 4;  // chunk flags (bits 0-2)
 
-// CTA barrier 0 returning whether any thread passed true.  The producer and the compute warps
-// reach it from their own loops, once per chunk each (a barrier counts warps, so the program
-// locations may differ between warps).
-__device__ __forceinline__ bool cta_any(bool pred)
-{
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 0, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)pred)
-        : "memory");
-    return r != 0;
-}
-
 // Items of one plan, (DM block fastest, time tile, part, group); CTA b takes b,
 // b + G, b + 2G, ...  kParts: the channels are cut into a->nsplit parts that add to the output, and
 // the item's first entry is its part.
@@ -1320,6 +1303,16 @@ bool packed_may_split(const StageGeom &g)
     return g.ngroups == 1 && !g.out_u16 && (g.out_i32 || g.nchans * most <= (1 << 24));
 }
 
+// Clocks of a launch of the generic kernel: 29, 24 or 18 adds a clock per SM with 32, 16 or 8 trials
+// a block (measured; fewer hide fewer waits), but a lone CTA takes 240 + 10 Db clocks a channel.
+double generic_clocks(const StageGeom &g)
+{
+    const double rate = g.Db >= 32 ? 29.0 : (g.Db >= 16 ? 24.0 : 18.0);
+    const double items = (double)g.ngroups * g.nblk * ((g.nsamp + g.T - 1) / g.T);
+    return g.nchans *
+           std::max(std::ceil(items / device_sms()) * g.Db * g.T / rate, 240.0 + 10.0 * g.Db);
+}
+
 }  // namespace
 
 // ---- fused batched launch: its tile shapes, tables and launch ----
@@ -1478,14 +1471,24 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
                 for (const auto &o : order)
                     if (kU8Shapes[o.second].tables(g, S, 2)) {
                         g.variant = o.second;
+                        g.est_clocks = o.first;
+                        g.may_split = packed_may_split(g);
                         return MDSM_OK;
                     }
             }
         }
         if ((g.in_dtype == MDSM_U16 || g.in_dtype == MDSM_I16) && !g.out_u16 &&
             (long long)g.nchans * 65535 <= 0x7fffffffLL &&
-            (packed_tables<CfgU16T<768>>(g, S, 3) || packed_tables<CfgU16T<512>>(g, S, 3)))
+            (packed_tables<CfgU16T<768>>(g, S, 3) || packed_tables<CfgU16T<512>>(g, S, 3))) {
+            const PackedShape &z = packed_shape_of(g);
+            const int sms = device_sms();
+            const double items = (double)g.nblk * ((g.nsamp + z.pt - 1) / z.pt) * g.ngroups;
+            g.may_split = packed_may_split(g);
+            g.est_clocks = packed_clocks(
+                z, g.ps, g.nchans, items,
+                g.may_split ? packed_split(z, g.ps, g.nchans, items, sms) : 1, sms);
             return MDSM_OK;
+        }
     }
     g.out_u16 = 0;  // only the uint8 packed kernel writes uint16 sums
     g.kernel = 1;
@@ -1513,7 +1516,10 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
             g.nst = 2;
             g.smem_bytes = smem_for(g);
         }
-        if (g.smem_bytes <= 200 * 1024) return MDSM_OK;
+        if (g.smem_bytes <= 200 * 1024) {
+            g.est_clocks = generic_clocks(g);
+            return MDSM_OK;
+        }
     }
     return fail(MDSM_EINVAL, "DM plan too wide for shared-memory staging (shift span " +
                                  std::to_string(g.max_span) + " per 8 DM trials)");
@@ -1570,6 +1576,12 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
         return fail(MDSM_EINVAL, "input row pitch must be a multiple of 16 bytes");
     if ((in_group_stride * SZ) % 16 != 0)
         return fail(MDSM_EINVAL, "input group pitch must be a multiple of 16 bytes");
+    if (g.gs.shape >= 0) {
+        MDSM_TRY(gs_launch(g, in, in_stride, out, out_stride, d_err, st, nsamp,
+                           mom && stage_folds_moments(g) ? mom : nullptr));
+        if (launches) *launches += 1;
+        return MDSM_OK;
+    }
     if (g.tm.shape >= 0) {
         MDSM_TRY(tm_launch(g, in, in_stride, in_group_stride, out, out_stride, out_group_stride,
                            d_err, st, nsamp));

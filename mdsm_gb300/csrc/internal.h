@@ -89,6 +89,22 @@ struct TmStage {
     size_t o_chunks = 0, o_chunk0 = 0, o_chan = 0;
 };
 
+// tables of a stage's group sums (groupsum.cu); shape -1: the stage has none
+struct GsStage {
+    int shape = -1;            // index of its kernel
+    int nblk = 0, DB = 0, T = 0;
+    int min_chunks = 0;        // chunks of the DM block that has the fewest
+    double block_clocks = 0;   // estimate of a DM block's tile
+    size_t smem = 0;
+    // host tables, until they are uploaded
+    std::vector<uint4> blobs;
+    std::vector<int4> chunks;
+    std::vector<int> chunk0;
+    std::vector<int2> chan;
+    void *d_tab = nullptr;     // blobs, then chunks, chunk0 and chan at these bytes
+    size_t o_chunks = 0, o_chunk0 = 0, o_chan = 0;
+};
+
 struct StageGeom {
     int nchans = 0;   // channels summed per group
     int ndms = 0;     // output rows per group
@@ -118,9 +134,11 @@ struct StageGeom {
                           // uint8, 3 packed uint16
     bool fill_sms = true; // the generic kernel's block may shrink to fill the SMs
     int variant = 0;      // packed uint8 kernel (not uint16 output): its tile shape
-    bool no_tm = false;   // never the tensor-memory form (the generic kernel asked for)
-    TmStage tm;           // where present it runs the stage; Db, T, kernel and the tables above
-                          // are those of the shared-memory kernels (batched launches, buffers)
+    bool fixed = false;   // the kernel or its block was asked for: neither of the forms below
+    bool may_split = false;  // its sums may be added up from parts of the channels
+    double est_clocks = 0;   // the chosen shared-memory kernel's estimate
+    TmStage tm;           // where present one of these runs the stage; Db, T, kernel and the tables
+    GsStage gs;           // above are those of the shared-memory kernels (batched launches, buffers)
 };
 
 // The tensor-memory form of a stage of float samples (tmsum.cu): its tables from the full shift table,
@@ -133,6 +151,14 @@ mdsm_status tm_launch(const StageGeom &g, const void *in, long long in_stride,
                       long long in_group_stride, void *out, long long out_stride,
                       long long out_group_stride, unsigned *d_err, cudaStream_t st,
                       long long nsamp);
+
+// The group sums of a stage of 8- or 16-bit samples (groupsum.cu), likewise.
+mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S);
+mdsm_status gs_upload(GsStage &t);
+void gs_release(GsStage &t);
+mdsm_status gs_launch(const StageGeom &g, const void *in, long long in_stride, void *out,
+                      long long out_stride, unsigned *d_err, cudaStream_t st, long long nsamp,
+                      unsigned long long *mom);
 
 // Build the blocked tables of a stage from a full shift table S[g][d][c] (row-major).  Picks
 // the tile shape: Db starts at 8*DPW (DPW as set on entry) and shrinks until the staged rows

@@ -185,12 +185,14 @@ mdsm_status plan_create_brute(const mdsm_brute_desc &d, Plan &p)
     g.DPW = d.dm_block == 16 ? 2 : (d.dm_block == 8 ? 1 : 4);
     g.kernel = d.kernel;
     g.fill_sms = d.dm_block == 0;
-    g.no_tm = d.kernel == 1 || d.dm_block != 0;
+    g.fixed = d.kernel == 1 || d.dm_block != 0;
     MDSM_TRY(build_stage_tables(g, p.S));
     MDSM_TRY(tm_build(g, p.S));
+    MDSM_TRY(gs_build(g, p.S));
     p.maxshift = g.max_shift;
     MDSM_TRY(upload_stage(g));
     MDSM_TRY(tm_upload(g.tm));
+    MDSM_TRY(gs_upload(g.gs));
     p.stages.push_back(std::move(g));
     p.in_stride = round_pitch((long long)p.nsamp + p.maxshift, p.in_dtype);
     return alloc_err(p);

@@ -115,6 +115,23 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// CTA barrier 0 returning whether any thread passed true.  The producer and the compute warps
+// reach it from their own loops, once per chunk each (a barrier counts warps, so the program
+// locations may differ between warps).
+__device__ __forceinline__ bool cta_any(bool pred)
+{
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 0, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)pred)
+        : "memory");
+    return r != 0;
+}
+
 // ------------------------------------------------------------------------------------------
 // Tensor memory (256 KB per SM: 128 lanes x 512 columns of 32 bits).  A warp reads and writes the
 // 32 lanes of its quarter (warp index mod 4); a .32x32b access moves one 32-bit column per

@@ -577,24 +577,15 @@ static void tm_offsets(const StageGeom &g, const std::vector<int32_t> &S, TmStag
         }
 }
 
-// The launch's estimated clocks in this form, and by the generic kernel (its block g.Db x g.T).
-// This one: 17.4 a trial and channel of a block, 1550 a chunk (its channels' last pairs, the waits) and
+// The launch's estimated clocks in this form: 17.4 a trial and channel of a block, 1550 a chunk (its channels' last pairs, the waits) and
 // an item, and the launch with its first chunks 15000; a least-squares fit to 240 launches (64-4096
 // channels, 32-3929 trials, 2295-250094 samples, spans of 0-130) with an rms error of 8%.
-// The generic one: 29, 24 or 18 adds a clock per SM with 32, 16 or 8 trials a block (measured; it
-// hides fewer waits), but a lone CTA takes 240 + 10 Db clocks a channel.
 static double tm_clocks(const StageGeom &g, const TmStage &t)
 {
     const double items = (double)g.ngroups * t.nblk;
     const double waves = std::ceil(items * ((g.nsamp + kTmT - 1) / kTmT) / device_sms());
     return waves * (17.4 * g.nchans * t.DB + 1550.0 * (double)t.chunks.size() / items + 1550.0) +
            15000.0;
-}
-static double generic_clocks(const StageGeom &g)
-{
-    const double rate = g.Db >= 32 ? 29.0 : (g.Db >= 16 ? 24.0 : 18.0);
-    const double items = (double)g.ngroups * ((g.ndms + g.Db - 1) / g.Db) * ((g.nsamp + g.T - 1) / g.T);
-    return g.nchans * std::max(std::ceil(items / device_sms()) * g.Db * g.T / rate, 240.0 + 10.0 * g.Db);
 }
 
 // Chooses among the shapes and the generic kernel by their estimates.  This form is taken where it is
@@ -605,9 +596,9 @@ static double generic_clocks(const StageGeom &g)
 mdsm_status tm_build(StageGeom &g, const std::vector<int32_t> &S)
 {
     tm_release(g.tm);
-    if (g.in_dtype != MDSM_F32 || g.no_tm) return MDSM_OK;
+    if (g.in_dtype != MDSM_F32 || g.fixed) return MDSM_OK;
     const std::vector<int2> ranges = tm_ranges(g, S);
-    double best = 0.85 * generic_clocks(g);
+    double best = 0.85 * g.est_clocks;
     TmStage pick;
     for (int i = 0; i < (int)(sizeof kTmShapes / sizeof kTmShapes[0]); ++i) {
         TmStage t;
