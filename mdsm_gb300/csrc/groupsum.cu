@@ -831,8 +831,10 @@ static int gs_split(const GsStage &t, double items)
 }
 
 // Chooses between the shapes and the shared-memory kernel that est_clocks is of by their estimates: this
-// form where it is estimated at 0.85 of the other's time or less (of 47 measured plans it took 18, at
-// 0.47-0.89 of the time; it loses where few channels make wide ones, whose trials hardly share patterns).
+// form where it is estimated at 0.9 (16-bit samples 0.85) of the other's time or less.  The uint8 kernels'
+// estimate lacks the launches, 16000 clocks; the 16-bit ones' is 8-16 % high instead.  Of 47 measured plans
+// it took 23, at 0.47-0.96 of the time; it loses where few channels make wide ones, whose trials hardly
+// share patterns.
 // f(0 .. n-1), each once, on up to eight threads.  An f that throws (no memory) is one that did nothing.
 template <class F>
 static void gs_parallel(int n, const F &f)
@@ -864,7 +866,7 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
         (long long)g.nchans * (sw == 1 ? 255 : 65535) > 0x7fffffffLL)
         return MDSM_OK;
     // the shape by its estimate over (some of) its DM blocks
-    double best = 0.85 * g.est_clocks;
+    double best = sw == 1 ? 0.9 * (g.est_clocks + 16000.0) : 0.85 * g.est_clocks;
     GsStage t;
     for (int i = 0; i < (int)(sizeof kGsShapes / sizeof kGsShapes[0]); ++i) {
         const GsShape &z = kGsShapes[i];
