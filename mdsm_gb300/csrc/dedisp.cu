@@ -237,6 +237,9 @@ struct PackedCfg {
     static constexpr int DB = NW * DPW;           // DM trials per tile
     static constexpr int DBS = (DB + 3) / 4 * 4;  // offsets per channel as stored (16-byte rows)
     static constexpr int THREADS = (NW + 1) * 32;
+    // no sample past the last output's is read (uint8: a plan's shape may be wider than another's;
+    // elsewhere the tile is read whole, 0.5 % faster for the short items of the subband stages)
+    static constexpr bool ENDS = SW == 1 && !U16OUT;
     static_assert(NW * 32 >= kPCC * DB, "the compute threads copy a chunk's offsets");
     static_assert(DPW == 1 || DPW == 2, "one or two DM trials per warp");
     static_assert(!U16OUT || SW == 1, "uint16 output from uint8 samples");
@@ -422,9 +425,9 @@ __device__ __forceinline__ void packed_stream(Src &src, unsigned char *smem, int
             if (lane < nc) {
                 const int c = c0 + lane;
                 const long long start = t0 + p_ss.x;
-                // (no sample past the last output's is read)
-                const long long end =
-                    start + min((long long)Cfg::PT, (long long)a.nsamp - t0) + p_ss.y;
+                long long len = Cfg::PT;
+                if constexpr (Cfg::ENDS) len = min(len, (long long)a.nsamp - t0);
+                const long long end = start + len + p_ss.y;
                 const long long sb = (start * SW) & ~15LL;  // bytes
                 const long long eb = (end * SW + 15) & ~15LL;
                 bytes = (unsigned)(eb - sb);
@@ -1556,7 +1559,7 @@ long long stage_in_bytes(const StageGeom &g, long long in_stride, long long in_g
 
 long long stage_reads(const StageGeom &g, long long in_stride, long long in_group_stride)
 {
-    if (g.kernel == 1) return stage_in_bytes(g, in_stride, in_group_stride);
+    if (g.kernel != 2 || g.out_u16) return stage_in_bytes(g, in_stride, in_group_stride);
     const long long SZ = (long long)dtype_size(g.in_dtype);
     return ((long long)(g.ngroups - 1) * in_group_stride + (long long)(g.nchans - 1) * in_stride) *
                SZ + (((long long)g.nsamp + g.max_shift) * SZ + 15) / 16 * 16;

@@ -168,7 +168,7 @@ mdsm_status upload_stage(StageGeom &g);
 void free_stage(StageGeom &g);
 // Bytes of input (from the group base) the kernel may read for in_stride, with tile overrun.
 long long stage_in_bytes(const StageGeom &g, long long in_stride, long long in_group_stride);
-// Bytes it does read: the packed kernels stop at the last output's last sample.
+// Bytes it does read: the packed uint8 kernels stop at the last output's last sample.
 long long stage_reads(const StageGeom &g, long long in_stride, long long in_group_stride);
 // Launch the stage kernel.  Returns number of kernels launched via *launches.
 // nsamp_run >= 0 computes only output samples [0, nsamp_run) (a time segment of the block,
