@@ -20,7 +20,7 @@
 // What bounds it: instruction issue (69 %), then shared memory (59 %): a pattern costs about 45 instructions
 // and 9 wavefronts a step, an add 2 and 1 a word.  4096 channels x 2^18 samples x 4096 trials: 206 ms by the
 // packed kernel (which is near its own bounds: 80 % shared memory, 70 % integer pipe), 132 ms here.  2048
-// channels of 16-bit samples x 30011 x 517: 3.09 -> 2.30 ms.  With one barrier a chunk and two buffers it
+// channels of 16-bit samples x 30011 x 517: 3.09 -> 2.14 ms.  With one barrier a chunk and two buffers it
 // took 188 ms; tasks of whole groups 206 (too few warps with a task); one word a lane and task 198 (decoding);
 // 19 warps of 3 trials 147, 11 of 6 135, five words a lane 154, four smaller buffers 146.
 #include <cuda_runtime.h>
@@ -43,7 +43,10 @@ namespace mdsm {
 namespace {
 
 constexpr int kGsT = 512;           // samples of a tile
-constexpr int kGsRaw = 3;           // stages of rows
+// Stages of rows: uint8 three (short parts want the copies' lead), 16-bit samples two half as large again
+// (their wider rows would leave chunks of one group; 2048 channels 2.29 -> 2.13 ms).
+__host__ __device__ constexpr int gs_raw(int sw) { return sw == 1 ? 3 : 2; }
+__host__ __device__ constexpr int gs_rawcap(int sw) { return 42 * 1024 / gs_raw(sw); }
 constexpr int kGsBlobs = 5;         // entries of tables: a chunk's are read until its sums are added
 constexpr int kGsZ = 3;             // pattern buffers
 constexpr int kGsRows = 32;         // channels of a chunk, at most
@@ -390,15 +393,16 @@ template <int SW, int NW, int DPW, bool SIGNED>
 __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_constant__ GsArgs a)
 {
     extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int RAW = gs_raw(SW);
     // a chunk's copies have landed / its patterns are stored (and its rows free) / its sums are added
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *built = full + kGsRaw, *added = built + kGsZ;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *built = full + RAW, *added = built + kGsZ;
     int4 *meta = reinterpret_cast<int4 *>(smem + 96);  // kGsBlobs: item, chunk bits, table bytes, flags
     unsigned char *blobs = smem + kGsHead;
     uint32_t *Z = reinterpret_cast<uint32_t *>(blobs + kGsBlobs * a.blobcap);
     unsigned char *raw = reinterpret_cast<unsigned char *>(Z + kGsZ * a.zcap);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int s = 0; s < kGsRaw; ++s) mbar_init(&full[s], 1);
+        for (int s = 0; s < RAW; ++s) mbar_init(&full[s], 1);
         for (int s = 0; s < kGsZ; ++s) {
             mbar_init(&built[s], NW);
             mbar_init(&added[s], NW);
@@ -440,7 +444,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_con
         };
         load();
         auto fill = [&](unsigned n) {  // chunk n of the stream
-            const int s = (int)(n % kGsRaw), e = (int)(n % kGsBlobs);
+            const int s = (int)(n % RAW), e = (int)(n % kGsBlobs);
             if (done) {
                 if (lane == 0) {
                     meta[e] = make_int4(-1, 0, 0, kGsStop);
@@ -477,19 +481,19 @@ __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_con
             ++k;
             load();
         };
-        for (unsigned n = 0; n < kGsRaw; ++n) fill(n);
+        for (unsigned n = 0; n < RAW; ++n) fill(n);
         for (unsigned k2 = 0;; ++k2) {
             if ((meta[k2 % kGsBlobs].w & kGsStop) != 0) return;  // (written by this warp)
             // chunk k2's rows are free, and the tables of chunk k2 - 2 (its sums were added before any
             // warp began with chunk k2's patterns)
             if (!gs_wait(&built[k2 % kGsZ], (k2 / kGsZ) & 1u, a.err)) {
                 // let the copies already issued land before the CTA exits (bounded as well)
-                for (unsigned q = k2; q < k2 + kGsRaw; ++q)
-                    mbar_wait_bounded(&full[q % kGsRaw], (q / kGsRaw) & 1u, nullptr, 0);
+                for (unsigned q = k2; q < k2 + RAW; ++q)
+                    mbar_wait_bounded(&full[q % RAW], (q / RAW) & 1u, nullptr, 0);
                 return;
             }
             fence_proxy_async_smem();
-            fill(k2 + kGsRaw);
+            fill(k2 + RAW);
         }
     }
 
@@ -500,8 +504,8 @@ __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_con
     // its share of chunk k's patterns; 0: done, 1: the stream has ended, -1: a wait ran out
     int first = warp;
     auto build = [&](unsigned k) {
-        const int s = (int)(k % kGsRaw), b = (int)(k % kGsZ);
-        if (!gs_wait(&full[s], (k / kGsRaw) & 1u, a.err)) return -1;
+        const int s = (int)(k % RAW), b = (int)(k % kGsZ);
+        if (!gs_wait(&full[s], (k / RAW) & 1u, a.err)) return -1;
         const int4 m = meta[k % kGsBlobs];
         if (m.w & kGsStop) return 1;
         if (k >= kGsZ && !gs_wait(&added[b], (k / kGsZ - 1) & 1u, a.err)) return -1;
@@ -565,12 +569,12 @@ const GsShape kGsShapes[] = {
 
 constexpr int kGsTrials = 72;  // trials of a block, at most
 constexpr int kGsShare = 8;    // tasks that a chunk aims at (3 and 14 measured 1-8% slower)
-constexpr int kGsRawCap = 14 * 1024, kGsBlobCap = 2 * 1024;
+constexpr int kGsBlobCap = 2 * 1024;
 constexpr int kGsZCap = 58 * 1024 / 4;  // words
 constexpr size_t kGsSmem = kGsHead + (size_t)kGsBlobs * kGsBlobCap + kGsZ * (size_t)kGsZCap * 4 +
-                           (size_t)kGsRaw * kGsRawCap;
+                           42 * 1024;
 static_assert(kGsSmem <= 227 * 1024, "shared memory");
-static_assert(kGsZCap < 65536 && kGsRawCap / 4 < 65536, "16-bit word offsets");
+static_assert(kGsZCap < 65536, "16-bit word offsets");
 
 // One group of channels for a block of trials: its distinct patterns (the channels' shifts relative to
 // the first's), in an order in which neighbours differ in few rows.
@@ -717,7 +721,7 @@ bool gs_fits(const GsShape &z, GsChunk &k, const GsGroup &q, const int2 *chan)
                        gs_pitch(sw, q, t.nseg, chan));
     t.pitch = (t.pitch + 15) / 16 * 16;
     if (t.rows > kGsRows || ng > kGsGroups || t.nseg > 31 || t.maxruns * t.nseg > kGsTasks || t.pitch > 255 * 16 ||
-        t.rows * t.pitch > kGsRawCap || t.npats * gs_row_words(sw, t.span) > kGsZCap ||
+        t.rows * t.pitch > gs_rawcap(sw) || t.npats * gs_row_words(sw, t.span) > kGsZCap ||
         16 * (t.maxruns * t.nseg + t.maxsteps) + 2 * gs_offsets(z.nw, z.dpw) * ng > kGsBlobCap)
         return false;
     k = t;
@@ -1055,7 +1059,7 @@ mdsm_status gs_launch(const StageGeom &g, const void *in, long long in_stride, v
     if (nitems > 0x7fffffffLL - 65536) return fail(MDSM_EINVAL, "block too long for one launch");
     a.ntiles = (int)ntiles;
     a.nitems = (int)nitems;
-    a.rawcap = kGsRawCap;
+    a.rawcap = gs_rawcap(z.sw);
     a.blobcap = kGsBlobCap;
     a.zcap = kGsZCap;
     a.out_i32 = g.out_i32;
