@@ -924,7 +924,8 @@ def main():
     hbm_achieved = alg_bytes / (per_launch_ms / 1e3) / 1e9
     traffic = None
     tp = os.path.join(ROOT, "profiles", "traffic.txt")
-    key = "packed" if info.kernel == 2 else "generic"
+    kern = plan.stage_info(0).kernel
+    key = {2: "packed", 5: "group_sums"}.get(kern, "generic")
     if os.path.exists(tp):
         for ln in open(tp):
             parts = ln.split()
@@ -950,8 +951,8 @@ def main():
                      "frac": achieved_ops / add_peak, "traffic": traffic,
                      "peak_source": "%d SMs x 128 lanes x sm_max_mhz (%s)" % (sm_count, pk_kind),
                      "kernel": {2: "k_shift_sum_packed<uint8>", 3: "k_shift_sum_packed<uint16>",
-                                4: "k_shift_sum_tm"}
-                     .get(info.kernel, "k_shift_sum"),
+                                4: "k_shift_sum_tm", 5: "k_group_sum<uint8>"}
+                     .get(kern, "k_shift_sum"),
                      "per_launch_ms": per_launch_ms,
                      "algorithmic_adds_per_launch": ops},
         "roofline_hbm": {"bound": "hbm", "achieved": hbm_achieved, "peak": pk.get("hbm_gbs"),

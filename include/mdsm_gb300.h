@@ -118,8 +118,8 @@ typedef struct {
     long long out_bytes;  /* ndms * nsamp * output element size                              */
     int in_dtype, out_dtype, acc;
     int dm_block, time_tile;
-    int kernel;           /* 1 generic, 2 packed 8-bit, 3 packed 16-bit, 4 float samples
-                             through tensor memory                                          */
+    int kernel;           /* 1 generic, 2 8-bit, 3 16-bit (packed, or by sums of groups of
+                             channels: see mdsm_stage_info), 4 float through tensor memory  */
     int nstages;          /* 1 brute force; subband: 2 per pass (mdsm_plan_stage_info)       */
     long long work_bytes; /* plan-owned device scratch (subband intermediate)               */
 } mdsm_plan_info;
@@ -135,7 +135,7 @@ void mdsm_plan_destroy(mdsm_plan *plan);
 mdsm_status mdsm_plan_get_info(const mdsm_plan *plan, mdsm_plan_info *info);
 
 /* One launch stage of a plan (brute force: stage 0; subband pass i: stages 2i and 2i+1): the
- * kernel it runs (as in mdsm_plan_info), its DM block and time tile,
+ * kernel it runs (as in mdsm_plan_info; 5 sums of groups of channels), its DM block and time tile,
  * and whether it writes uint16 subband series. */
 typedef struct {
     int kernel, dm_block, time_tile, out_u16;

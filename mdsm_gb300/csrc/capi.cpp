@@ -242,7 +242,7 @@ mdsm_status mdsm_plan_stage_info(const mdsm_plan *plan, int stage, mdsm_stage_in
     const StageGeom &g = p.stages[(size_t)stage];
     std::memset(info, 0, sizeof(*info));
     const bool tm = g.tm.shape >= 0, gs = g.gs.shape >= 0;
-    info->kernel = tm ? 4 : g.kernel;
+    info->kernel = tm ? 4 : gs ? 5 : g.kernel;
     info->dm_block = tm ? g.tm.DB : gs ? g.gs.DB : g.Db;
     info->time_tile = tm ? g.tm.T : gs ? g.gs.T : g.T;
     info->out_u16 = g.out_u16;

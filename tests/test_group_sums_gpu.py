@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SMEM = 231680  # of the kernel's shared memory: no other kernel's
+GROUPS = 5  # mdsm_stage_info's kernel
 SEEN = set()
 PLANS = [  # type, nchans, nsamp, segments, bandwidth
     ("u8", 1203, 9000, [(0.0, 0.23, 181)], 100.0),
@@ -30,9 +30,9 @@ def test_group_sums(lib, orc, cuda, dtype, nchans, nsamp, segs, bw, out_dtype):
     plan = m.BrutePlan(nchans, 1500.0, -bw / nchans, 64e-6, nsamp, segs, in_dtype=dtype,
                        out_dtype=out_dtype)
     i, st = plan.info, plan.stage_info(0)
-    if out_dtype == "f32" and dtype != "u8" and st.smem_bytes != SMEM:
+    if out_dtype == "f32" and dtype != "u8" and st.kernel != GROUPS:
         pytest.skip("float parts would not be exact: whole tiles are too few, or summed in floats")
-    assert st.smem_bytes == SMEM
+    assert st.kernel == GROUPS
     SEEN.add((dtype, i.dm_block))
     np_t = {"u8": np.uint8, "u16": np.uint16, "i16": np.int16}[dtype]
     lo, hi = np.iinfo(np_t).min, np.iinfo(np_t).max
@@ -68,7 +68,7 @@ def test_group_sums_fold_moments(lib, orc, cuda):
     from mdsm_gb300.serving import Server
     nchans, nsamp, segs = 801, 20000, [(0.0, 0.23, 300)]
     plan = m.BrutePlan(nchans, 1500.0, -100.0 / nchans, 64e-6, nsamp, segs, out_dtype="i32")
-    assert plan.stage_info(0).smem_bytes == SMEM
+    assert plan.stage_info(0).kernel == GROUPS
     srv = Server(max_inflight=1, nwidths=7, threshold=6.0, cand_cap=4096)
     b = srv.add_beam(nchans, 1500.0, -100.0 / nchans, 64e-6, nsamp, segs)
     x = synth.gaussian_u8(nchans, nsamp + srv.beam_info(b).maxshift, 5)
