@@ -81,7 +81,8 @@ __device__ __forceinline__ float sum_as_double(const float (&x)[B])
 }
 
 // Sums of B = 2, 4 or 8 samples on 16-byte aligned rows: a thread reads the samples of 16 bytes
-// of output (or of 4 outputs) as 16-byte pieces.
+// of output (or of 4 outputs) as 16-byte pieces.  Bound by DRAM: float 1024 x 2^15 by 2 and by 4 in
+// 37 us each (83 and 72 % of the copy rate); one double sum a thread (FP64 pipe 86 %) took 490 together.
 template <typename TIn, typename TOut, int B>
 __global__ void __launch_bounds__(256)
     k_downsample_sum(const TIn *__restrict__ in, long long in_stride, long long nout,

@@ -839,9 +839,9 @@ static int gs_split(const GsStage &t, double items)
 // estimate lacks the launches, 16000 clocks; the 16-bit ones' is 8-16 % high instead.  Of 47 measured plans
 // it took 23, at 0.47-0.96 of the time; it loses where few channels make wide ones, whose trials hardly
 // share patterns.
-// f(0 .. n-1), each once, on up to eight threads.  An f that throws (no memory) is one that did nothing.
+// f(0 .. n-1), each once, on up to eight threads (one for a small table, which a thread costs more than).  An f that throws (no memory) is one that did nothing.
 template <class F>
-static void gs_parallel(int n, const F &f)
+static void gs_parallel(int n, size_t table, const F &f)
 {
     std::atomic<int> next(0);
     auto work = [&]() {
@@ -853,7 +853,7 @@ static void gs_parallel(int n, const F &f)
         }
     };
     std::vector<std::thread> pool;
-    const int most = std::min({8, (int)std::thread::hardware_concurrency(), n / 2});
+    const int most = table < (1u << 18) ? 1 : std::min({8, (int)std::thread::hardware_concurrency(), n / 2});
     try {
         for (int k = 1; k < most; ++k) pool.emplace_back(work);
     } catch (...) {  // (no more threads: fewer do it)
@@ -878,7 +878,7 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
         const int DB = z.db(), nblk = (g.ndms + DB - 1) / DB, step = (nblk + 7) / 8;
         const int n = (nblk + step - 1) / step;
         std::vector<std::pair<double, int>> seen((size_t)n, {-1.0, 0});  // clocks, chunks
-        gs_parallel(n, [&](int k) {
+        gs_parallel(n, S.size(), [&](int k) {
             std::vector<int2> chan((size_t)g.nchans);
             std::vector<GsGroup> groups;
             std::vector<GsChunk> chunks;
@@ -919,7 +919,7 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
         bool ok = false;
     };
     std::vector<Block> blocks((size_t)t.nblk);
-    gs_parallel(t.nblk, [&](int b) {
+    gs_parallel(t.nblk, S.size(), [&](int b) {
         std::vector<GsGroup> groups;
         std::vector<GsChunk> chunks;
         Block &o = blocks[(size_t)b];
