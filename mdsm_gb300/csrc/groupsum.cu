@@ -411,10 +411,12 @@ __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_con
     }
     __syncthreads();
 
-    // item: DM block fastest, then the time tile, then the part of the channels
+    // item: DM block fastest (from tile to tile a different one first, so that a CTA does not meet the
+    // same block, perhaps the costliest, in each of its items), then the time tile, then the part of the
+    // channels
     auto chunks_of = [&](int it, int &blk, int &tile) {
-        blk = it % a.nblk;
         const int rest = it / a.nblk;
+        blk = (int)(((unsigned)it + (unsigned)rest) % (unsigned)a.nblk);
         tile = rest % a.ntiles;
         const int part = rest / a.ntiles;
         const int k0 = __ldg(a.chunk0 + blk), n = __ldg(a.chunk0 + blk + 1) - k0;
@@ -813,11 +815,12 @@ void gs_release(GsStage &t)
     t = GsStage();
 }
 
-// Clocks of a launch over `items` tiles, each cut into `split` parts of the channels.
+// Clocks of a launch over `items` tiles, each cut into `split` parts of the channels; the last of the
+// waves may be of the costliest blocks.
 static double gs_clocks(const GsStage &t, double items, int split, int sms)
 {
-    return std::ceil(items * split / sms) * (t.block_clocks / split + kGsShapes[t.shape].item) +
-           11000.0 + (split > 1 ? 5000.0 : 0.0);
+    return (std::ceil(items * split / sms) - 1.0) * (t.block_clocks / split + kGsShapes[t.shape].item) +
+           t.most_clocks / split + kGsShapes[t.shape].item + 11000.0 + (split > 1 ? 5000.0 : 0.0);
 }
 static int gs_split(const GsStage &t, double items)
 {
@@ -885,12 +888,13 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
             if (gs_block(g, S, z, k * step * DB, chan.data(), groups, chunks))
                 seen[(size_t)k] = {gs_block_clocks(z, groups, chunks), (int)chunks.size()};
         });
-        double clk = 0;
+        double clk = 0, most = 0;
         int least = INT32_MAX;
         bool ok = true;
         for (const auto &v : seen) {
             ok = ok && v.first >= 0;
             clk += v.first;
+            most = std::max(most, v.first);
             least = std::min(least, v.second);
         }
         if (!ok) continue;
@@ -900,6 +904,7 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
         u.DB = DB;
         u.T = kGsT;
         u.block_clocks = clk / n;
+        u.most_clocks = most;
         u.min_chunks = least;
         const double items = (double)nblk * ((g.nsamp + kGsT - 1) / kGsT);
         const double c = gs_clocks(u, items, g.may_split ? gs_split(u, items) : 1, device_sms());
@@ -1000,6 +1005,7 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
         }
         t.chunk0.push_back((int)t.chunks.size());
         t.block_clocks += o.clk / t.nblk;
+        t.most_clocks = std::max(t.most_clocks, o.clk);
         t.min_chunks = std::min(t.min_chunks, (int)o.chunks.size());
     }
     t.smem = kGsSmem;

@@ -94,7 +94,7 @@ struct GsStage {
     int shape = -1;            // index of its kernel
     int nblk = 0, DB = 0, T = 0;
     int min_chunks = 0;        // chunks of the DM block that has the fewest
-    double block_clocks = 0;   // estimate of a DM block's tile
+    double block_clocks = 0, most_clocks = 0;  // estimate of a DM block's tile: mean, largest
     size_t smem = 0;
     // host tables, until they are uploaded
     std::vector<uint4> blobs;

@@ -165,12 +165,19 @@ __device__ __forceinline__ void tm_main(TmAcc<C> &acc, uint32_t tb, const uint16
     }
 }
 
+// The item's DM block: fastest, and from tile to tile a different one first, so that a CTA does not meet
+// the same block, perhaps the costliest, in each of its items.
+__device__ __forceinline__ int tm_block(const TmArgs &a, int item, int rest)
+{
+    return (int)(((unsigned)item + (unsigned)rest) % (unsigned)a.nblk);
+}
+
 // Stores the item's rows of this warp.
 template <class C>
 __device__ __forceinline__ void tm_store(const TmArgs &a, const TmAcc<C> &acc, int item, int q, int tg,
                                          int lane)
 {
-    const int blk = item % a.nblk, rest = item / a.nblk;
+    const int rest = item / a.nblk, blk = tm_block(a, item, rest);
     const int tile = rest % a.ntiles, g = rest / a.ntiles;
     const long long t0 = (long long)tile * kTmT + (32 * q + lane) * kTmL;
 #pragma unroll
@@ -342,7 +349,7 @@ __global__ void __launch_bounds__(kTmThreads, 1)
             }
         };
         for (int it = blockIdx.x; it < a.nitems && !late; it += gridDim.x) {
-            const int blk = it % a.nblk, rest = it / a.nblk;
+            const int rest = it / a.nblk, blk = tm_block(a, it, rest);
             const int tile = rest % a.ntiles, g = rest / a.ntiles;
             const long long t0 = (long long)tile * kTmT;
             const int cnt = (int)min((long long)kTmT, (long long)a.nsamp - t0);
@@ -584,8 +591,10 @@ static double tm_clocks(const StageGeom &g, const TmStage &t)
 {
     const double items = (double)g.ngroups * t.nblk;
     const double waves = std::ceil(items * ((g.nsamp + kTmT - 1) / kTmT) / device_sms());
-    return waves * (17.4 * g.nchans * t.DB + 1550.0 * (double)t.chunks.size() / items + 1550.0) +
-           15000.0;
+    int most = 0;  // (the last wave may be of the blocks with the most chunks)
+    for (size_t b = 0; b + 1 < t.chunk0.size(); ++b) most = std::max(most, t.chunk0[b + 1] - t.chunk0[b]);
+    return waves * (17.4 * g.nchans * t.DB + 1550.0) +
+           1550.0 * ((waves - 1.0) * (double)t.chunks.size() / items + most) + 15000.0;
 }
 
 // Chooses among the shapes and the generic kernel by their estimates.  This form is taken where it is
