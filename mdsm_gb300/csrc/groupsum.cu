@@ -30,6 +30,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <thread>
 #include <type_traits>
 #include <utility>
@@ -866,7 +867,7 @@ static void gs_parallel(int n, size_t table, const F &f)
 }
 
 mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
-{
+try {
     gs_release(g.gs);
     const int sw = (int)dtype_size(g.in_dtype);
     if (g.fixed || g.ngroups != 1 || g.out_u16 || !g.acc_int || sw > 2 ||
@@ -1011,6 +1012,9 @@ mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
     t.smem = kGsSmem;
     g.gs = std::move(t);
     return MDSM_OK;
+} catch (const std::bad_alloc &) {  // (no memory for these tables on the host either)
+    gs_release(g.gs);
+    return MDSM_OK;
 }
 
 mdsm_status gs_upload(GsStage &t)
@@ -1019,7 +1023,11 @@ mdsm_status gs_upload(GsStage &t)
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t b0 = up(t.blobs.size() * 16), b1 = up(t.chunks.size() * sizeof(int4));
     const size_t b2 = up(t.chunk0.size() * 4), b3 = up(t.chan.size() * sizeof(int2));
-    MDSM_CUDA_TRY(cudaMalloc(&t.d_tab, b0 + b1 + b2 + b3));
+    if (cudaMalloc(&t.d_tab, b0 + b1 + b2 + b3) != cudaSuccess) {
+        cudaGetLastError();  // (no memory for these tables: the packed kernel runs the stage)
+        t = GsStage();
+        return MDSM_OK;
+    }
     char *d = static_cast<char *>(t.d_tab);
     t.o_chunks = b0;
     t.o_chunk0 = b0 + b1;

@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 
 #include "box.cuh"
 #include "internal.h"
@@ -603,7 +604,7 @@ static double tm_clocks(const StageGeom &g, const TmStage &t)
 // wide (1 MHz channels at 1.2 GHz, steps of 1 pc cm^-3: 12 samples a block and more; a chunk is then
 // two or three channels) and where there are too few tiles of 1536 samples to fill the SMs.
 mdsm_status tm_build(StageGeom &g, const std::vector<int32_t> &S)
-{
+try {
     tm_release(g.tm);
     if (g.in_dtype != MDSM_F32 || g.fixed) return MDSM_OK;
     const std::vector<int2> ranges = tm_ranges(g, S);
@@ -622,6 +623,9 @@ mdsm_status tm_build(StageGeom &g, const std::vector<int32_t> &S)
     tm_offsets(g, S, pick);
     g.tm = std::move(pick);
     return MDSM_OK;
+} catch (const std::bad_alloc &) {  // (no memory for these tables on the host either)
+    tm_release(g.tm);
+    return MDSM_OK;
 }
 
 mdsm_status tm_upload(TmStage &t)
@@ -630,7 +634,11 @@ mdsm_status tm_upload(TmStage &t)
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t b0 = up(t.offs.size() * 2), b1 = up(t.chunks.size() * sizeof(int4));
     const size_t b2 = up(t.chunk0.size() * 4), b3 = up(t.chan.size() * sizeof(int2));
-    MDSM_CUDA_TRY(cudaMalloc(&t.d_tab, b0 + b1 + b2 + b3));
+    if (cudaMalloc(&t.d_tab, b0 + b1 + b2 + b3) != cudaSuccess) {
+        cudaGetLastError();  // (no memory for these tables: the generic kernel runs the stage)
+        t = TmStage();
+        return MDSM_OK;
+    }
     char *d = static_cast<char *>(t.d_tab);
     MDSM_CUDA_TRY(cudaMemcpy(d, t.offs.data(), t.offs.size() * 2, cudaMemcpyHostToDevice));
     MDSM_CUDA_TRY(cudaMemcpy(d + b0, t.chunks.data(), t.chunks.size() * sizeof(int4),
