@@ -606,7 +606,8 @@ static double tm_clocks(const StageGeom &g, const TmStage &t)
 mdsm_status tm_build(StageGeom &g, const std::vector<int32_t> &S)
 try {
     tm_release(g.tm);
-    if (g.in_dtype != MDSM_F32 || g.fixed) return MDSM_OK;
+    // (int32 output is converted by the generic kernel's store; this one stores floats)
+    if (g.in_dtype != MDSM_F32 || g.out_i32 || g.fixed) return MDSM_OK;
     const std::vector<int2> ranges = tm_ranges(g, S);
     double best = 0.85 * g.est_clocks;
     TmStage pick;
