@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <utility>
 
 #include "clip.cuh"
 #include "cutsum.cuh"
@@ -260,6 +261,9 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
     constexpr int SPW = 4 / (int)sizeof(T);  // samples per word
     constexpr int N = 4 * SPW;               // columns of a vector
     cg::cluster_group cl = cg::this_cluster();
+    // (the wait comes before the first store to another CTA's memory, which may only be touched
+    // once that CTA is known to run; the loads and sums between hide it)
+    auto started = cl.barrier_arrive();
     const int rank = (int)cl.block_rank(), nrank = (int)cl.num_blocks();
     const int tid = threadIdx.x, half = tid & 1;
     const long long t0 = (long long)(blockIdx.x / nrank) * (2 * N) + half * N;
@@ -377,6 +381,7 @@ __global__ void __launch_bounds__(kSpecThreads, 2)
         }
     }
     __syncthreads();
+    cl.barrier_wait(std::move(started));
     if (tid < 2 * N) {
         long long s1 = 0;
         unsigned long long s2 = 0;
