@@ -25,13 +25,14 @@ __device__ __forceinline__ uint32_t special_key(float x)
 // 2^(E-26) and u3 = 2^(E-41); cutting with a constant C = 1.5 * 2^23 units rounds to the unit
 // (for a sample below 2^22 of the first), so the second and third hold at most half a unit of
 // the one before (1024 of them stay within 2^24 units: exact adds), and the first is watched.
-// What a rare small sample leaves past the third is added exactly beside them, and its lowest
-// bit noted.  While the first's sums stay below 2^23 u1 and 2^53 lowest bits, every partial sum
-// is a whole number of lowest bits below 2^53: the double sum is exact at every step, in any
+// What a rare small sample leaves past the third is added exactly beside them, and its lowest bit
+// noted (it is looked for in the bits of what each sample leaves: a float sum of those would absorb
+// the smaller ones).  While the first's sums stay below 2^23 u1 and 2^53 lowest bits, every partial
+// sum is a whole number of lowest bits below 2^53: the double sum is exact at every step, in any
 // order.  Otherwise (ok() false) the caller sums in double.  15 float operations a sample
 // against one at the double rate (64 clocks of a scheduler for a warp).
 struct CutSum {
-    float c1, c2, c3, a1, a2, a3, a4, left, seen, top, unit;
+    float c1, c2, c3, a1, a2, a3, a4, top, unit;
     __device__ __forceinline__ void start(float biggest)
     {
         // 2^E as a float, 0 (no cut fits) for zero, tiny, huge or special values
@@ -41,7 +42,7 @@ struct CutSum {
         c2 = p * (1.5f / 8.0f);      // 1.5 * 2^(23 + E - 26)
         c3 = p * (1.5f / 262144.0f); // 1.5 * 2^(23 + E - 41)
         unit = c3 * (1.0f / 12582912.0f);
-        a1 = a2 = a3 = a4 = left = seen = top = 0.0f;
+        a1 = a2 = a3 = a4 = top = 0.0f;
     }
     // the thirds of x; returns what is left past them
     __device__ __forceinline__ float cut(float x, float &h1, float &h2, float &h3) const
@@ -56,18 +57,18 @@ struct CutSum {
     template <int U>
     __device__ __forceinline__ void add(const float (&v)[U])
     {
+        uint32_t left = 0u;
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             float h1, h2, h3;
-            const float r3 = cut(v[j], h1, h2, h3);
+            left |= __float_as_uint(cut(v[j], h1, h2, h3));
             a1 = __fadd_rn(a1, h1);
             a2 = __fadd_rn(a2, h2);
             a3 = __fadd_rn(a3, h3);
-            left = __fadd_rn(left, fabsf(r3));
             top = fmaxf(top, fmaxf(fabsf(a1), __fadd_rn(fabsf(v[j]), fabsf(v[j]))));
         }
-        if (left == seen) return;
-        // some sample of these left a part past the third (or is not finite: left turns NaN)
+        if ((left & 0x7fffffffu) == 0u) return;  // (-0 leaves -0)
+        // some sample of these left a part past the third (or is not finite, and leaves a NaN)
 #pragma unroll 1
         for (int j = 0; j < U; ++j) {
             float x = v[0];
@@ -85,12 +86,12 @@ struct CutSum {
             unit = err == 0.0f && low > 0.0f ? fminf(unit, low) : 0.0f;
             a4 = s;
         }
-        seen = left;
     }
+    __device__ __forceinline__ bool finite() const { return a1 == a1 && top < INFINITY; }
     __device__ __forceinline__ bool ok() const
     {
         // (2^53 lowest bits as 2^29 of them times 2^24; NaN and infinities fail a comparison)
-        return c1 > 0.0f && left < INFINITY && top < c1 * 0.66f &&
+        return c1 > 0.0f && finite() && top < c1 * 0.66f &&
                top * (1.01f / 536870912.0f) < unit * 16777216.0f;
     }
     __device__ __forceinline__ double sum() const

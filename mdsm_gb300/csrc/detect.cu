@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kRefThreads)
     }
     // the warps' sums: the thirds as whole numbers of their units
     long long i1 = 0, i2 = 0, i3 = 0;
-    const bool ok = cs.c1 > 0.0f && cs.left < INFINITY && cs.top < cs.c1 * 0.66f;
+    const bool ok = cs.c1 > 0.0f && cs.finite() && cs.top < cs.c1 * 0.66f;
     if (ok) {
         i1 = __float2ll_rn(cs.a1 / u1);
         i2 = __float2ll_rn(cs.a2 / u2);
