@@ -27,9 +27,10 @@ __device__ __forceinline__ uint32_t special_key(float x)
 // the one before (1024 of them stay within 2^24 units: exact adds), and the first is watched.
 // What a rare small sample leaves past the third is added exactly beside them, and its lowest bit
 // noted (it is looked for in the bits of what each sample leaves: a float sum of those would absorb
-// the smaller ones).  While the first's sums stay below 2^23 u1 and 2^53 lowest bits, every partial
-// sum is a whole number of lowest bits below 2^53: the double sum is exact at every step, in any
-// order.  Otherwise (ok() false) the caller sums in double.  15 float operations a sample
+// the smaller ones).  While the first's sums stay below 2^23 u1, and with what the others can hold
+// (512 u1 and less) below 2^53 lowest bits, every partial sum is a whole number of lowest bits below
+// 2^53: the double sum is exact at every step, in any order.  Otherwise (ok() false) the caller sums
+// in double.  15 float operations a sample
 // against one at the double rate (64 clocks of a scheduler for a warp).
 struct CutSum {
     float c1, c2, c3, a1, a2, a3, a4, top, unit;
@@ -90,9 +91,11 @@ struct CutSum {
     __device__ __forceinline__ bool finite() const { return a1 == a1 && top < INFINITY; }
     __device__ __forceinline__ bool ok() const
     {
+        // a partial sum: the first third's (at most top), 1024 halves of u1, of u2 and of u3 (513 u1)
+        const float most = __fadd_rn(top, c1 * (513.0f / 12582912.0f));
         // (2^53 lowest bits as 2^29 of them times 2^24; NaN and infinities fail a comparison)
         return c1 > 0.0f && finite() && top < c1 * 0.66f &&
-               top * (1.01f / 536870912.0f) < unit * 16777216.0f;
+               most * (1.01f / 536870912.0f) < unit * 16777216.0f;
     }
     __device__ __forceinline__ double sum() const
     {

@@ -19,10 +19,15 @@ def _rows():
         for at, v in put:
             x[at] = v
         rows.append(x)
+    x = np.zeros(1024, np.float32)  # partial sums past 2^53 lowest bits by the small samples alone
+    x[[0, 4, 8, 12]] = 1.0, 1.0, 1.0, 0.9375
+    x[[20, 600]] = 2.0 ** -51
+    x[32:512] = 2.0 ** -12 - 2.0 ** -26
+    rows.append(x)
     return rows
 
 
-@pytest.mark.parametrize("k", range(4))
+@pytest.mark.parametrize("k", range(5))
 @pytest.mark.parametrize("axis", ["channels", "spectra"])
 def test_clip_of_cancelling_samples(lib, orc, cuda, k, axis):
     import mdsm_gb300 as m
@@ -37,7 +42,7 @@ def test_clip_of_cancelling_samples(lib, orc, cuda, k, axis):
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
-@pytest.mark.parametrize("k", range(4))
+@pytest.mark.parametrize("k", range(5))
 def test_block_statistics_of_cancelling_samples(lib, orc, cuda, k):
     import mdsm_gb300 as m
     r = _rows()[k]

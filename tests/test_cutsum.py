@@ -1,7 +1,7 @@
 """The exact float sums of the RFI clip's and the detector's statistics (mdsm_gb300/csrc/cutsum.cuh),
 compiled for the host: where they say that they are exact, they equal the left-to-right double sum bit for
 bit.  Ordinary data has to be summed exactly; data with remainders past the third cut, cancelling sums,
-infinities and NaN may only be declined."""
+partial sums at the edge of 53 bits, infinities and NaN may only be declined."""
 import ctypes
 import os
 import subprocess
@@ -71,6 +71,17 @@ REMAINDERS = [
 @pytest.mark.parametrize("k", range(len(REMAINDERS)))
 def test_small_remainders_are_not_dropped(cut_sum, k):
     _check(cut_sum, REMAINDERS[k])
+
+
+def test_partial_sums_beyond_53_bits_are_declined(cut_sum):
+    """The first third's sum stays below 2^53 lowest bits, the sum of the second takes it past them:
+    the chain loses a lowest bit at 4.0 and another after it."""
+    x = np.zeros(1024, np.float32)
+    x[[0, 4, 8, 12]] = 1.0, 1.0, 1.0, 0.9375
+    x[20] = 2.0 ** -51
+    x[32:512] = 2.0 ** -12 - 2.0 ** -26
+    x[600] = 2.0 ** -51
+    _check(cut_sum, x)
 
 
 def test_cancelling_samples_of_many_sizes(cut_sum):
