@@ -598,6 +598,18 @@ static double tm_clocks(const StageGeom &g, const TmStage &t)
            1550.0 * ((waves - 1.0) * (double)t.chunks.size() / items + most) + 15000.0;
 }
 
+// Whether a shape's kernel came out at the registers whose shares it deals out (its increase would wait for
+// ever on fewer).
+static bool tm_built(const TmShape &z)
+{
+    cudaFuncAttributes at;
+    if (cudaFuncGetAttributes(&at, z.fn) != cudaSuccess) {
+        cudaGetLastError();  // (the generic kernel runs the stage)
+        return false;
+    }
+    return at.numRegs == kTmRegs;
+}
+
 // Chooses among the shapes and the generic kernel by their estimates.  This form is taken where it is
 // estimated at 0.85 of the generic kernel's time or less, which leaves room for the error of both: of
 // 97 measured plans it took 56, at 0.44-0.97 of the generic kernel's time.  It loses where spans are
@@ -613,7 +625,7 @@ try {
     TmStage pick;
     for (int i = 0; i < (int)(sizeof kTmShapes / sizeof kTmShapes[0]); ++i) {
         TmStage t;
-        if (!tm_tables(g, ranges, i, t)) continue;
+        if (!tm_built(kTmShapes[i]) || !tm_tables(g, ranges, i, t)) continue;
         const double clk = tm_clocks(g, t);
         if (clk < best) {
             best = clk;
@@ -664,10 +676,6 @@ mdsm_status tm_launch(const StageGeom &g, const void *in, long long in_stride,
 {
     const TmStage &t = g.tm;
     const TmShape &z = kTmShapes[t.shape];
-    cudaFuncAttributes at;
-    MDSM_CUDA_TRY(cudaFuncGetAttributes(&at, z.fn));
-    if (at.numRegs != kTmRegs)  // (the register shares would not add up)
-        return fail(MDSM_ECUDA, "tensor-memory kernel: built with unexpected registers");
     MDSM_CUDA_TRY(cudaFuncSetAttribute(z.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)t.smem));
     const char *d = static_cast<const char *>(t.d_tab);
