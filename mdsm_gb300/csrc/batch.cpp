@@ -297,12 +297,16 @@ void drop_graph(mdsm_batch *b)
     b->graph_choice = -1;
 }
 
+// What the launches' times depend on: the beams' sizes and, since a launch per beam is one of the choices, the
+// kernel and tile of each beam's own launch (a line of another form, or of other kernels, does not match).
 std::string geometry_key(const mdsm_batch *b)
 {
     std::ostringstream k;
+    k << "v2:";
     for (mdsm_plan *p : b->plans) {
         const StageGeom &g = p->p.stages[0];
         k << g.nchans << "x" << g.ndms << "x" << g.nsamp << "k" << g.kernel << "s" << g.max_span
+          << "b" << g.Db << "t" << g.T << "p" << g.variant << "g" << g.gs.shape << "f" << g.tm.shape
           << ";";
     }
     return k.str();
