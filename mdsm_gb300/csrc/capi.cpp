@@ -227,7 +227,7 @@ mdsm_status mdsm_plan_get_info(const mdsm_plan *plan, mdsm_plan_info *info)
         const bool tm = g.tm.shape >= 0, gs = g.gs.shape >= 0;
         info->dm_block = tm ? g.tm.DB : gs ? g.gs.DB : g.Db;
         info->time_tile = tm ? g.tm.T : gs ? g.gs.T : g.T;
-        info->kernel = tm ? 4 : g.kernel;
+        info->kernel = tm ? 4 : gs ? (dtype_size(g.in_dtype) == 1 ? 2 : 3) : g.kernel;
     }
     info->nstages = (int)p.stages.size();
     info->work_bytes = (long long)p.work_bytes;
