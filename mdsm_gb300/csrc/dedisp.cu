@@ -1476,8 +1476,12 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
                 std::sort(order.begin(), order.end());
                 for (const auto &o : order)
                     if (kU8Shapes[o.second].tables(g, S, 2)) {
+                        const PackedShape &z = kU8Shapes[o.second];
+                        const double items =
+                            (double)g.nblk * ((g.nsamp + z.pt - 1) / z.pt) * g.ngroups;
                         g.variant = o.second;
                         g.est_clocks = o.first;
+                        g.est_whole = packed_clocks(z, g.ps, g.nchans, items, 1, sms);
                         g.may_split = packed_may_split(g);
                         return MDSM_OK;
                     }
@@ -1490,6 +1494,7 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
             const int sms = device_sms();
             const double items = (double)g.nblk * ((g.nsamp + z.pt - 1) / z.pt) * g.ngroups;
             g.may_split = packed_may_split(g);
+            g.est_whole = packed_clocks(z, g.ps, g.nchans, items, 1, sms);
             g.est_clocks = packed_clocks(
                 z, g.ps, g.nchans, items,
                 g.may_split ? packed_split(z, g.ps, g.nchans, items, sms) : 1, sms);
@@ -1523,7 +1528,7 @@ mdsm_status build_stage_tables(StageGeom &g, const std::vector<int32_t> &S)
             g.smem_bytes = smem_for(g);
         }
         if (g.smem_bytes <= 200 * 1024) {
-            g.est_clocks = generic_clocks(g);
+            g.est_clocks = g.est_whole = generic_clocks(g);
             return MDSM_OK;
         }
     }
@@ -1582,9 +1587,10 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
         return fail(MDSM_EINVAL, "input row pitch must be a multiple of 16 bytes");
     if ((in_group_stride * SZ) % 16 != 0)
         return fail(MDSM_EINVAL, "input group pitch must be a multiple of 16 bytes");
-    if (g.gs.shape >= 0) {
-        MDSM_TRY(gs_launch(g, in, in_stride, out, out_stride, d_err, st, nsamp,
-                           mom && stage_folds_moments(g) ? mom : nullptr));
+    // (a store that folds moments has whole sums: parts would each have some of them)
+    if (!stage_folds_moments(g)) mom = nullptr;
+    if (g.gs.shape >= 0 && (!mom || g.gs.whole)) {
+        MDSM_TRY(gs_launch(g, in, in_stride, out, out_stride, d_err, st, nsamp, mom));
         if (launches) *launches += 1;
         return MDSM_OK;
     }
@@ -1600,7 +1606,6 @@ mdsm_status launch_stage(const StageGeom &g, const void *in, long long in_stride
     const long long ntiles = (nsamp + g.T - 1) / g.T;
     long long nitems = (long long)g.nblk * ntiles * g.ngroups;
     const int sms = device_sms();
-    if (!(mom && stage_folds_moments(g))) mom = nullptr;
     int nsplit = 1;
     if (g.kernel == 3 || (g.kernel == 2 && !g.out_u16)) {
         const PackedShape &z = packed_shape_of(g);

@@ -874,7 +874,8 @@ try {
         (long long)g.nchans * (sw == 1 ? 255 : 65535) > 0x7fffffffLL)
         return MDSM_OK;
     // the shape by its estimate over (some of) its DM blocks
-    double best = sw == 1 ? 0.9 * (g.est_clocks + 16000.0) : 0.85 * g.est_clocks;
+    auto limit = [&](double other) { return sw == 1 ? 0.9 * (other + 16000.0) : 0.85 * other; };
+    double best = limit(g.est_clocks);
     GsStage t;
     for (int i = 0; i < (int)(sizeof kGsShapes / sizeof kGsShapes[0]); ++i) {
         const GsShape &z = kGsShapes[i];
@@ -1010,6 +1011,11 @@ try {
         t.min_chunks = std::min(t.min_chunks, (int)o.chunks.size());
     }
     t.smem = kGsSmem;
+    // A launch that folds moments has one part, and may be slower than the packed kernel's where the choice
+    // fell for the parts: the same rule again, for one part of both (1734 channels x 3852 samples x 575 trials:
+    // 331 us against 238; 192 x 3396 x 25: 46 against 29; whole tiles enough, 801 x 20000 x 300: 281, 329).
+    t.whole = gs_clocks(t, (double)t.nblk * ((g.nsamp + kGsT - 1) / kGsT), 1, device_sms()) <
+              limit(g.est_whole);
     g.gs = std::move(t);
     return MDSM_OK;
 } catch (const std::bad_alloc &) {  // (no memory for these tables on the host either)

@@ -94,6 +94,7 @@ struct GsStage {
     int shape = -1;            // index of its kernel
     int nblk = 0, DB = 0, T = 0;
     int min_chunks = 0;        // chunks of the DM block that has the fewest
+    bool whole = true;         // also where the channels may not be cut into parts
     double block_clocks = 0, most_clocks = 0;  // estimate of a DM block's tile: mean, largest
     size_t smem = 0;
     // host tables, until they are uploaded
@@ -137,6 +138,7 @@ struct StageGeom {
     bool fixed = false;   // the kernel or its block was asked for: neither of the forms below
     bool may_split = false;  // its sums may be added up from parts of the channels
     double est_clocks = 0;   // the chosen shared-memory kernel's estimate
+    double est_whole = 0;    // the same with the channels not cut into parts
     TmStage tm;           // where present one of these runs the stage; Db, T, kernel and the tables
     GsStage gs;           // above are those of the shared-memory kernels (batched launches, buffers)
 };
