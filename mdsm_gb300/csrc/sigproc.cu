@@ -69,8 +69,9 @@ mdsm_status pack_u8_rows(const float *in, long long in_stride, int nrows, long l
     return MDSM_OK;
 }
 
-// Any channel count and alignment: one CTA moves a tile of 32 spectra x 32 channels: loads walk channels
-// (consecutive in the raw stream), stores walk time (consecutive in the output rows).
+// Any channel count and alignment, 4 bits a sample and more: one CTA moves a tile of 32 spectra x 32
+// channels: loads walk channels (consecutive in the raw stream), stores walk time (consecutive in
+// the output rows).
 template <int NBITS, typename TOut>
 __global__ void __launch_bounds__(256)
     k_unpack_transpose(const uint8_t *__restrict__ raw, long long nspectra, int nchans, int invert,
@@ -100,9 +101,8 @@ __global__ void __launch_bounds__(256)
                 memcpy(&f, raw + 4 * idx, 4);
                 v = (TOut)f;
             } else {
-                const long long bit = idx * NBITS;
-                const unsigned b = raw[bit >> 3];
-                v = (TOut)((b >> (bit & 7)) & ((1u << NBITS) - 1u));
+                static_assert(NBITS == 4, "smaller samples take k_unpack_tile");
+                v = (TOut)((raw[idx >> 1] >> (4 * (idx & 1))) & 15u);
             }
         }
         tile[ty + 8 * i][tx] = v;
@@ -258,19 +258,20 @@ static void unpack_go(const uint8_t *raw, long long nspectra, int nchans, int in
                       long long out_stride, long long col0, cudaStream_t st)
 {
     TOut *o = static_cast<TOut *>(out);
-    const int align = NBITS >= 2 ? NBITS / 2 : 1;  // bytes of 4 samples
-    if (nchans % (NBITS == 1 ? 8 : 4) == 0 && ((uintptr_t)raw % (uintptr_t)align) == 0) {
-        constexpr int TT = 128 / (int)sizeof(TOut);
-        const int vec = (((uintptr_t)o | (uintptr_t)(out_stride * (long long)sizeof(TOut)) |
-                          (uintptr_t)(col0 * (long long)sizeof(TOut))) & 15) == 0;
-        dim3 grid((unsigned)((nspectra + TT - 1) / TT), (unsigned)((nchans + 127) / 128));
-        k_unpack_tile<NBITS, TOut><<<grid, 256, 0, st>>>(raw, nspectra, nchans, invert, o,
-                                                         out_stride, col0, vec);
-    } else {
-        dim3 grid((unsigned)((nspectra + 31) / 32), (unsigned)((nchans + 31) / 32));
-        k_unpack_transpose<NBITS, TOut><<<grid, dim3(32, 8), 0, st>>>(raw, nspectra, nchans, invert,
-                                                                      o, out_stride, col0);
-    }
+    // (spectra of 1- and 2-bit samples are whole bytes, so whole groups of channels)
+    if constexpr (NBITS > 2)
+        if (nchans % 4 != 0 || (uintptr_t)raw % (uintptr_t)(NBITS / 2) != 0) {  // bytes of 4 samples
+            dim3 grid((unsigned)((nspectra + 31) / 32), (unsigned)((nchans + 31) / 32));
+            k_unpack_transpose<NBITS, TOut><<<grid, dim3(32, 8), 0, st>>>(
+                raw, nspectra, nchans, invert, o, out_stride, col0);
+            return;
+        }
+    constexpr int TT = 128 / (int)sizeof(TOut);
+    const int vec = (((uintptr_t)o | (uintptr_t)(out_stride * (long long)sizeof(TOut)) |
+                      (uintptr_t)(col0 * (long long)sizeof(TOut))) & 15) == 0;
+    dim3 grid((unsigned)((nspectra + TT - 1) / TT), (unsigned)((nchans + 127) / 128));
+    k_unpack_tile<NBITS, TOut><<<grid, 256, 0, st>>>(raw, nspectra, nchans, invert, o, out_stride,
+                                                     col0, vec);
 }
 
 template <int NBITS>
