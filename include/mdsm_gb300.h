@@ -169,7 +169,9 @@ mdsm_status mdsm_subband_shift_tables(const mdsm_subband_desc *desc, int pass, i
  * d_out: [ndms] rows of out_stride elements.  Replaces call_dedisperse's kernel dispatch
  * (src/mdsm/dedispersion_wrapper.cu:7-9 -> dedispersion_thread.cu:332-341).  Asynchronous on
  * stream: a device-side wait that ran out (the kernels' waits are bounded; the block's results
- * are then invalid) is reported by the next mdsm_plan_check. */
+ * are then invalid) is reported by the next mdsm_plan_check.  The kernels take (nearly) all shared memory
+ * of the SMs they run on: a kernel of the caller's that waits on the device for this call's
+ * results has to leave SMs free of its blocks. */
 mdsm_status mdsm_dedisperse_device(mdsm_plan *plan, const void *d_in, long long in_stride,
                                    size_t in_bytes, void *d_out, long long out_stride,
                                    void *stream);

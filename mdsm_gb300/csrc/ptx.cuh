@@ -139,8 +139,8 @@ __device__ __forceinline__ bool cta_any(bool pred)
 // ------------------------------------------------------------------------------------------
 constexpr uint32_t kTmemCols = 512;
 
-// One warp allocates all columns (waits while another CTA of the SM holds them); the base
-// address is written to *slot in shared memory.
+// One warp allocates all columns (waits, without a bound, while another CTA of the SM holds any: the caller
+// sees to it that none is there); the base address is written to *slot in shared memory.
 __device__ __forceinline__ void tmem_alloc_all(uint32_t *slot)
 {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(

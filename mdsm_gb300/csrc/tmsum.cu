@@ -437,15 +437,17 @@ struct TmShape {
 const TmShape kTmShapes[] = {TM(4), TM(3), TM(2)};
 #undef TM
 
+// Each launch asks for all of a CTA's shared memory.  With the 1 KB that the system keeps per CTA that is all
+// the SM has, so a CTA gets an SM that no other CTA (of any kernel) is on or comes to: the tensor memory is
+// free, and its allocation, the one wait here that has no bound, does not wait.
 constexpr size_t kTmSmem = 227 * 1024;
 
+// Bytes that a ring of nst chunks needs of it.
 size_t tm_smem(int nst, int ncmax, int rowcap, int db)
 {
     const int ncpad = (ncmax + kTmPad - 1) / kTmPad * kTmPad;
-    const size_t b = kTmHead + (kTmEntries * kTmMeta + 127) / 128 * 128 +
-                     (size_t)nst * ncmax * rowcap + 128 +
-                     (size_t)kTmEntries * (tm_offbytes(db, ncpad) + 16);
-    return std::max<size_t>(b, 120 * 1024);  // (one CTA a SM: it holds all tensor memory)
+    return kTmHead + (kTmEntries * kTmMeta + 127) / 128 * 128 + (size_t)nst * ncmax * rowcap + 128 +
+           (size_t)kTmEntries * (tm_offbytes(db, ncpad) + 16);
 }
 
 }  // namespace
@@ -550,7 +552,7 @@ static bool tm_tables(const StageGeom &g, const std::vector<int2> &ranges, int s
     // a ring of at least three chunks, more where they fit: short chunks need the lead
     t.nst = 3;
     while (t.nst < kTmStages && tm_smem(t.nst + 1, ncmax, t.rowcap, DB) <= kTmSmem) ++t.nst;
-    t.smem = tm_smem(t.nst, ncmax, t.rowcap, DB);
+    t.smem = kTmSmem;
     t.noff = noff;
     return true;
 }

@@ -1,5 +1,5 @@
 // Whether a plan's float stage takes the tensor-memory kernel, where the runtime reports `argv[1]` registers
-// a thread for it (0: it reports an error): prints the chosen shape, -1 for none.
+// a thread for it (0: it reports an error): prints the chosen shape, -1 for none, and its shared memory.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -23,9 +23,9 @@ int main(int argc, char **argv)
     g_regs = argc > 1 ? std::atoi(argv[1]) : 0;
     mdsm::StageGeom g;
     g.nchans = 128;
-    g.ndms = 496;
+    g.ndms = argc > 2 ? std::atoi(argv[2]) : 496;
     g.ngroups = 1;
-    g.nsamp = 32000;
+    g.nsamp = argc > 3 ? std::atoi(argv[3]) : 32000;
     g.in_dtype = MDSM_F32;
     g.acc_int = 0;
     g.DPW = 4;
@@ -33,6 +33,6 @@ int main(int argc, char **argv)
     for (int d = 0; d < g.ndms; ++d)
         for (int c = 0; c < g.nchans; ++c) S[(size_t)d * g.nchans + c] = d * c / 512;
     if (mdsm::build_stage_tables(g, S) != MDSM_OK || mdsm::tm_build(g, S) != MDSM_OK) return 1;
-    std::printf("%d\n", g.tm.shape);
+    std::printf("%d %zu\n", g.tm.shape, g.tm.smem);
     return 0;
 }

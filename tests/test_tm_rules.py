@@ -1,5 +1,10 @@
-"""The tensor-memory kernel shares out the registers that it is launched with; a build in which it does not
-come out at exactly these is not used, and its stages keep the generic kernel (no call fails for it)."""
+"""The rules by which a float stage takes the tensor-memory kernel, compiled for the host.
+
+The tensor-memory kernel shares out the registers that it is launched with; a build in which it does not
+come out at exactly these is not used, and its stages keep the generic kernel (no call fails for it).
+
+Its allocation of an SM's tensor memory would wait, without a bound, for another kernel's CTA that holds some
+there, so it asks for so much shared memory that it shares its SMs with no other CTA."""
 import os
 import platform
 import re
@@ -23,13 +28,26 @@ def rules(lib, tmp_path_factory):
                     os.path.join(ROOT, "tests", "drivers", "tm_rules.cu"), *objs, "-o", exe,
                     "-lpthread"], check=True, capture_output=True)
 
-    def f(regs):
-        return int(subprocess.run([exe, str(regs)], check=True, capture_output=True, text=True).stdout)
+    def f(*args):
+        r = subprocess.run([exe, *map(str, args)], check=True, capture_output=True, text=True)
+        return tuple(map(int, r.stdout.split()))
     return f
 
 
+REGS = int(re.search(r"kTmRegs = (\d+)", open(os.path.join(CSRC, "tmsum.cu")).read()).group(1))
+SMEM_PER_SM = 228 * 1024  # bytes of shared memory per SM (sm_100 family)
+SMEM_PER_CTA_RESERVED = 1024
+
+
 def test_other_register_counts_keep_the_generic_kernel(rules):
-    regs = int(re.search(r"kTmRegs = (\d+)", open(os.path.join(CSRC, "tmsum.cu")).read()).group(1))
-    assert rules(regs) >= 0
-    for other in (0, regs - 8, regs + 8):
-        assert rules(other) == -1
+    assert rules(REGS)[0] >= 0
+    for other in (0, REGS - 8, REGS + 8):
+        assert rules(other)[0] == -1
+
+
+@pytest.mark.parametrize("ndms,nsamp", [(496, 32000), (96, 200000), (2000, 9000)])
+def test_no_other_cta_on_its_sms(rules, ndms, nsamp):
+    shape, smem = rules(REGS, ndms, nsamp)
+    assert shape >= 0
+    left = SMEM_PER_SM - (smem + SMEM_PER_CTA_RESERVED)
+    assert 0 <= left < SMEM_PER_CTA_RESERVED
