@@ -594,9 +594,8 @@ struct GsGroup {
 
 int popc_bytes(uint64_t x)  // bytes that are not zero
 {
-    int n = 0;
-    for (; x; x >>= 8) n += (x & 255) != 0;
-    return n;
+    const uint64_t low = 0x7f7f7f7f7f7f7f7full;
+    return __builtin_popcountll(((x & low) + low | x) & ~low);
 }
 
 // s: the block's first trial's shifts, nd trials of `stride` channels.
@@ -612,16 +611,23 @@ void gs_group(const int32_t *s, int nd, long long stride, int c0, int n, GsGroup
         lo[i] = INT32_MAX;
         hi[i] = INT32_MIN;
     }
-    for (int d = 0; d < nd; ++d) {
-        const int32_t *v = s + d * stride + c0;
-        lo0 = std::min(lo0, v[0]);
-        hi0 = std::max(hi0, v[0]);
-        for (int i = 0; i < n; ++i) {
-            rel[d][i] = v[i] - v[0];
-            lo[i] = std::min(lo[i], rel[d][i]);
-            hi[i] = std::max(hi[i], rel[d][i]);
+    auto ranges = [&](auto count) {  // (whole groups: a fixed count, which the compiler vectorises)
+        const int m = count;
+        for (int d = 0; d < nd; ++d) {
+            const int32_t *v = s + d * stride + c0;
+            lo0 = std::min(lo0, v[0]);
+            hi0 = std::max(hi0, v[0]);
+            for (int i = 0; i < m; ++i) {
+                rel[d][i] = v[i] - v[0];
+                lo[i] = std::min(lo[i], rel[d][i]);
+                hi[i] = std::max(hi[i], rel[d][i]);
+            }
         }
-    }
+    };
+    if (n == kGsG)
+        ranges(std::integral_constant<int, kGsG>());
+    else
+        ranges(n);
     q.smin = lo0;
     q.span = hi0 - lo0;
     for (int i = 0; i < n; ++i) {
@@ -744,19 +750,22 @@ double gs_cut(const GsShape &z, const int32_t *s, int nd, long long stride, int 
         fits = gs_row_off(sw, q, i, ch.x) * sw >= -kGsPad;
     }
     const double add = gs_add_waves(z);
-    double cost = 0;
+    double cost = 0, least = 0;
     if (fits) {
         GsChunk k;
         fits = gs_fits(z, k, q, chan);
         cost = gs_build_waves(sw, q, k.nseg) + add;
+        // what a half takes at least: its rows once, one pattern, the adds
+        least = gs_nseg(sw, 0) * (9.0 * ((n / 2 + 1) / 2) + (sw == 1 ? 13.0 : 6.0)) + add;
     }
-    if (n == 1 || (fits && cost < 2 * add)) {
+    if (n == 1 || (fits && cost <= 2 * least)) {
         out.push_back(std::move(q));
         return fits ? cost : -1;
     }
     std::vector<GsGroup> a;
     const double l = gs_cut(z, s, nd, stride, c0, n / 2, chan, a);
-    const double r = l < 0 ? -1 : gs_cut(z, s, nd, stride, c0 + n / 2, n - n / 2, chan, a);
+    const double r = l < 0 || (fits && cost <= l + least)
+                         ? -1 : gs_cut(z, s, nd, stride, c0 + n / 2, n - n / 2, chan, a);
     if (r < 0 && !fits) return -1;
     if (r < 0 || (fits && cost <= l + r)) {
         out.push_back(std::move(q));
@@ -838,12 +847,8 @@ static int gs_split(const GsStage &t, double items)
     return best;
 }
 
-// Chooses between the shapes and the shared-memory kernel that est_clocks is of by their estimates: this
-// form where it is estimated at 0.9 (16-bit samples 0.85) of the other's time or less.  The uint8 kernels'
-// estimate lacks the launches, 16000 clocks; the 16-bit ones' is 8-16 % high instead.  Of 47 measured plans
-// it took 23, at 0.47-0.96 of the time; it loses where few channels make wide ones, whose trials hardly
-// share patterns.
-// f(0 .. n-1), each once, on up to eight threads (one for a small table, which a thread costs more than).  An f that throws (no memory) is one that did nothing.
+// f(0 .. n-1), each once, on up to eight threads (one for a table so small that a thread costs more).  An f
+// that throws (no memory) is one that did nothing.
 template <class F>
 static void gs_parallel(int n, size_t table, const F &f)
 {
@@ -857,7 +862,7 @@ static void gs_parallel(int n, size_t table, const F &f)
         }
     };
     std::vector<std::thread> pool;
-    const int most = table < (1u << 18) ? 1 : std::min({8, (int)std::thread::hardware_concurrency(), n / 2});
+    const int most = table < (1u << 13) ? 1 : std::min({8, (int)std::thread::hardware_concurrency(), n});
     try {
         for (int k = 1; k < most; ++k) pool.emplace_back(work);
     } catch (...) {  // (no more threads: fewer do it)
@@ -866,6 +871,11 @@ static void gs_parallel(int n, size_t table, const F &f)
     for (auto &p : pool) p.join();
 }
 
+// Chooses between the shapes and the shared-memory kernel that est_clocks is of by their estimates: this
+// form where it is estimated at 0.9 (16-bit samples 0.85) of the other's time or less.  The uint8 kernels'
+// estimate lacks the launches, 16000 clocks; the 16-bit ones' is 8-16 % high instead.  Of 47 measured plans
+// it took 23, at 0.47-0.96 of the time; it loses where few channels make wide ones, whose trials hardly
+// share patterns.
 mdsm_status gs_build(StageGeom &g, const std::vector<int32_t> &S)
 try {
     gs_release(g.gs);
@@ -876,64 +886,92 @@ try {
     // the shape by its estimate over (some of) its DM blocks
     auto limit = [&](double other) { return sw == 1 ? 0.9 * (other + 16000.0) : 0.85 * other; };
     double best = limit(g.est_clocks);
-    GsStage t;
+    struct Block {  // a DM block's tables in the making
+        std::vector<int2> chan;
+        std::vector<GsGroup> groups;
+        std::vector<GsChunk> chunks;
+        double clk = 0;
+        bool ok = false;
+        void form(const StageGeom &g, const std::vector<int32_t> &S, const GsShape &z, int d0)
+        {
+            chan.resize((size_t)g.nchans);
+            if (!gs_block(g, S, z, d0, chan.data(), groups, chunks)) return;
+            clk = gs_block_clocks(z, groups, chunks);
+            ok = true;
+        }
+    };
+    struct Sampled {  // a shape, its number of blocks, and every step-th of them
+        int shape, nblk, step;
+        std::vector<Block> seen;
+    };
+    std::vector<Sampled> shapes;
+    std::vector<std::pair<int, int>> work;
     for (int i = 0; i < (int)(sizeof kGsShapes / sizeof kGsShapes[0]); ++i) {
         const GsShape &z = kGsShapes[i];
         if (z.sw != sw || (z.sgn != 0) != (g.in_dtype == MDSM_I16)) continue;
-        const int DB = z.db(), nblk = (g.ndms + DB - 1) / DB, step = (nblk + 7) / 8;
+        const int nblk = (g.ndms + z.db() - 1) / z.db(), step = (nblk + 7) / 8;
         const int n = (nblk + step - 1) / step;
-        std::vector<std::pair<double, int>> seen((size_t)n, {-1.0, 0});  // clocks, chunks
-        gs_parallel(n, S.size(), [&](int k) {
-            std::vector<int2> chan((size_t)g.nchans);
-            std::vector<GsGroup> groups;
-            std::vector<GsChunk> chunks;
-            if (gs_block(g, S, z, k * step * DB, chan.data(), groups, chunks))
-                seen[(size_t)k] = {gs_block_clocks(z, groups, chunks), (int)chunks.size()};
-        });
+        for (int k = 0; k < n; ++k) work.emplace_back((int)shapes.size(), k);
+        shapes.push_back({i, nblk, step, std::vector<Block>((size_t)n)});
+    }
+    gs_parallel((int)work.size(), S.size(), [&](int w) {
+        Sampled &u = shapes[(size_t)work[(size_t)w].first];
+        const int k = work[(size_t)w].second;
+        const GsShape &z = kGsShapes[u.shape];
+        u.seen[(size_t)k].form(g, S, z, k * u.step * z.db());
+    });
+    GsStage t;
+    Sampled *from = nullptr;
+    for (Sampled &v : shapes) {
         double clk = 0, most = 0;
         int least = INT32_MAX;
         bool ok = true;
-        for (const auto &v : seen) {
-            ok = ok && v.first >= 0;
-            clk += v.first;
-            most = std::max(most, v.first);
-            least = std::min(least, v.second);
+        for (const Block &o : v.seen) {
+            ok = ok && o.ok;
+            clk += o.clk;
+            most = std::max(most, o.clk);
+            least = std::min(least, (int)o.chunks.size());
         }
         if (!ok) continue;
         GsStage u;
-        u.shape = i;
-        u.nblk = nblk;
-        u.DB = DB;
+        u.shape = v.shape;
+        u.nblk = v.nblk;
+        u.DB = kGsShapes[v.shape].db();
         u.T = kGsT;
-        u.block_clocks = clk / n;
+        u.block_clocks = clk / (double)v.seen.size();
         u.most_clocks = most;
         u.min_chunks = least;
-        const double items = (double)nblk * ((g.nsamp + kGsT - 1) / kGsT);
+        const double items = (double)u.nblk * ((g.nsamp + kGsT - 1) / kGsT);
         const double c = gs_clocks(u, items, g.may_split ? gs_split(u, items) : 1, device_sms());
         if (c < best) {
             best = c;
             t = u;
+            from = &v;
         }
     }
     if (t.shape < 0) return MDSM_OK;
     const GsShape &z = kGsShapes[t.shape];
     t.chan.resize((size_t)t.nblk * g.nchans);
-    // the tables, DM block by DM block, on a few threads
-    struct Block {
+    // the tables, DM block by DM block, on a few threads (the blocks that were looked at are there)
+    struct Table {
         std::vector<uint4> blobs;
         std::vector<int4> chunks;
         double clk = 0;
         bool ok = false;
     };
-    std::vector<Block> blocks((size_t)t.nblk);
+    std::vector<Table> tables((size_t)t.nblk);
     gs_parallel(t.nblk, S.size(), [&](int b) {
-        std::vector<GsGroup> groups;
-        std::vector<GsChunk> chunks;
-        Block &o = blocks[(size_t)b];
+        Block made;
+        Block &src = b % from->step == 0 ? from->seen[(size_t)(b / from->step)] : made;
+        Table &o = tables[(size_t)b];
         const int d0 = b * t.DB, nd = std::min(g.ndms - d0, t.DB);
+        if (!src.ok) src.form(g, S, z, d0);
+        if (!src.ok) return;
         int2 *ch = &t.chan[(size_t)b * g.nchans];
-        if (!gs_block(g, S, z, d0, ch, groups, chunks)) return;
-        o.clk = gs_block_clocks(z, groups, chunks);
+        std::copy(src.chan.begin(), src.chan.end(), ch);
+        const std::vector<GsGroup> &groups = src.groups;
+        const std::vector<GsChunk> &chunks = src.chunks;
+        o.clk = src.clk;
         for (const GsChunk &k : chunks) {
             const int ng = (int)(k.g1 - k.g0), rw = gs_row_words(sw, k.span);
             // the groups' patterns in runs, so that about kGsShare warps have a task (each run starts
@@ -997,7 +1035,7 @@ try {
     });
     t.chunk0.push_back(0);
     t.block_clocks = 0;
-    for (const Block &o : blocks) {
+    for (const Table &o : tables) {
         const size_t at = t.blobs.size();
         if (!o.ok || at + o.blobs.size() > 0x7fffffffu) return MDSM_OK;
         t.blobs.insert(t.blobs.end(), o.blobs.begin(), o.blobs.end());
