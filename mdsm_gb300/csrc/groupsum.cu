@@ -7,11 +7,11 @@
 // per group where the packed kernels add one per channel.  Integer sums do not depend on their order.
 //
 // One CTA: NW warps of DPW trials each x 512 samples, and a warp that copies.  The channels come in chunks
-// of a few groups: rows by bulk copies, three chunks ahead, with the chunk's tables.  The compute warps
-// take tasks (a segment of a run of patterns): the run's first pattern adds the group's rows, each further
-// one swaps the rows in which it differs (gs_patterns).  Then each adds the patterns for its trials
-// (gs_add).  A warp works on chunk k + 1's tasks before it adds chunk k, over three pattern buffers, so
-// warps without a task, or with a longer one, do not hold the others up at a barrier.
+// of a few groups: rows by bulk copies, three chunks ahead (16-bit samples two), with the chunk's tables.
+// The compute warps take tasks (a segment of a run of patterns): the run's first pattern adds the group's
+// rows, each further one swaps the rows in which it differs (gs_patterns).  Then each adds the patterns for
+// its trials (gs_add).  A warp works on chunk k + 1's tasks before it adds chunk k, over three pattern
+// buffers, so warps without a task, or with a longer one, do not hold the others up at a barrier.
 //
 // Groups of 8, 4, 2 or 1 channels are chosen where the tables are made, by the wavefronts that they take:
 // 8 where a block's trials share patterns well (4096 channels, steps of 0.24 pc cm^-3), 4 and less where
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, 1) k_group_sum(const __grid_con
     };
 
     if (warp == NW) {
-        // ---- the copies, three chunks ahead, across items ----
+        // ---- the copies, RAW chunks ahead, across items ----
         int it = (int)blockIdx.x - (int)gridDim.x, blk = 0, tile = 0, k = 0;
         int2 ks = make_int2(0, 0);
         int4 ck = make_int4(0, 0, 0, 0);

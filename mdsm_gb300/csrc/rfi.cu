@@ -10,10 +10,11 @@
 //
 // The double operations of the clip test are the slow pipe of this GPU (2 lanes per clock per
 // SM), so a row's test is turned once into two bounds of the sample type (clip.cuh) and the
-// samples are compared as integers or floats; the float statistics keep the two double
-// operations a sample that their rounding needs (FP64 pipe 50-55 % busy: what bounds them).
-// uint8 4096 x 97921: 137 us the channels, 249 the spectra; before, with the test in double and one
-// thread a spectrum, 2330 and 3003.  Float 1001 x 40003: 231 and 164 us; before 662 and 976.
+// samples are compared as integers or floats; the float statistics keep one double operation a
+// sample, the multiply-add of the squares (FP64 pipe 56-59 % busy: what bounds them), and sum the
+// samples themselves exactly in float (cutsum.cuh).
+// uint8 4096 x 97921: 138 us the channels, 252 the spectra; before, with the test in double and one
+// thread a spectrum, 2330 and 3003.  Float 1001 x 40003: 230 and 145 us; before 662 and 976.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

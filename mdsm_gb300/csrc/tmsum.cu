@@ -331,87 +331,87 @@ __global__ void __launch_bounds__(kTmThreads, 1)
         // ---- the copies (the last warpgroup's first warp) ----
         regs_fewer<kTmRegsCopy>();
         if (warp == kTmMain + kTmFill) {
-        unsigned s = 0, round = 0, n = 0;  // chunk n's rows go to stage s, round `round` of the ring
-        bool late = false;
-        // waits for stage s and chunk n's entry to be free again
-        auto claim = [&]() {
-            if (round > 0 && !warp_wait(&empty[s], (round - 1) & 1u, a.err)) return false;
-            if (n >= kTmEntries &&
-                !warp_wait(&used[n & (kTmEntries - 1)], (n / kTmEntries - 1) & 1u, a.err))
-                return false;
-            fence_proxy_async_smem();
-            return true;
-        };
-        auto next_stage = [&]() {
-            ++n;
-            if (++s == nst) {
-                s = 0;
-                ++round;
-            }
-        };
-        for (int it = blockIdx.x; it < a.nitems && !late; it += gridDim.x) {
-            const int rest = it / a.nblk, blk = tm_block(a, it, rest);
-            const int tile = rest % a.ntiles, g = rest / a.ntiles;
-            const long long t0 = (long long)tile * kTmT;
-            const int cnt = (int)min((long long)kTmT, (long long)a.nsamp - t0);
-            const int gb = g * a.nblk + blk;
-            const int2 *chan = a.chan + (size_t)gb * a.nchans;
-            const unsigned char *in_g = a.in + (size_t)(g * a.in_group_stride) * 4;
-            const int k0 = __ldg(a.chunk0 + gb), k1 = __ldg(a.chunk0 + gb + 1);
-            int4 ck = __ldg(a.chunks + k0);
-            int2 ch = lane < ck.y ? __ldg(chan + ck.x + lane) : make_int2(0, 0);
-            for (int k = k0; k < k1; ++k) {
-                // the next chunk's entries are loaded before this one waits for its stage
-                const int4 nk = k + 1 < k1 ? __ldg(a.chunks + k + 1) : make_int4(0, 0, 0, 0);
-                const int2 nch = lane < nk.y ? __ldg(chan + nk.x + lane) : make_int2(0, 0);
-                if (!claim()) {
-                    late = true;
-                    break;
+            unsigned s = 0, round = 0, n = 0;  // chunk n's rows go to stage s, round `round` of the ring
+            bool late = false;
+            // waits for stage s and chunk n's entry to be free again
+            auto claim = [&]() {
+                if (round > 0 && !warp_wait(&empty[s], (round - 1) & 1u, a.err)) return false;
+                if (n >= kTmEntries &&
+                    !warp_wait(&used[n & (kTmEntries - 1)], (n / kTmEntries - 1) & 1u, a.err))
+                    return false;
+                fence_proxy_async_smem();
+                return true;
+            };
+            auto next_stage = [&]() {
+                ++n;
+                if (++s == nst) {
+                    s = 0;
+                    ++round;
                 }
-                unsigned char *entry = meta + (n & (kTmEntries - 1)) * kTmMeta;
-                unsigned bytes = 0;
-                const unsigned char *src = nullptr;
-                if (lane < ck.y) {
-                    const long long start = t0 + ch.x;
-                    const long long end = start + cnt + ((unsigned)ch.y >> 16);
-                    const long long sb = (start * 4) & ~15LL;
-                    const long long eb = (end * 4 + 15) & ~15LL;
-                    bytes = (unsigned)(eb - sb);
-                    src = in_g + (size_t)(ck.x + lane) * (size_t)a.in_stride * 4 + sb;
-                    reinterpret_cast<int *>(entry + 16)[lane] = ch.y;
+            };
+            for (int it = blockIdx.x; it < a.nitems && !late; it += gridDim.x) {
+                const int rest = it / a.nblk, blk = tm_block(a, it, rest);
+                const int tile = rest % a.ntiles, g = rest / a.ntiles;
+                const long long t0 = (long long)tile * kTmT;
+                const int cnt = (int)min((long long)kTmT, (long long)a.nsamp - t0);
+                const int gb = g * a.nblk + blk;
+                const int2 *chan = a.chan + (size_t)gb * a.nchans;
+                const unsigned char *in_g = a.in + (size_t)(g * a.in_group_stride) * 4;
+                const int k0 = __ldg(a.chunk0 + gb), k1 = __ldg(a.chunk0 + gb + 1);
+                int4 ck = __ldg(a.chunks + k0);
+                int2 ch = lane < ck.y ? __ldg(chan + ck.x + lane) : make_int2(0, 0);
+                for (int k = k0; k < k1; ++k) {
+                    // the next chunk's entries are loaded before this one waits for its stage
+                    const int4 nk = k + 1 < k1 ? __ldg(a.chunks + k + 1) : make_int4(0, 0, 0, 0);
+                    const int2 nch = lane < nk.y ? __ldg(chan + nk.x + lane) : make_int2(0, 0);
+                    if (!claim()) {
+                        late = true;
+                        break;
+                    }
+                    unsigned char *entry = meta + (n & (kTmEntries - 1)) * kTmMeta;
+                    unsigned bytes = 0;
+                    const unsigned char *src = nullptr;
+                    if (lane < ck.y) {
+                        const long long start = t0 + ch.x;
+                        const long long end = start + cnt + ((unsigned)ch.y >> 16);
+                        const long long sb = (start * 4) & ~15LL;
+                        const long long eb = (end * 4 + 15) & ~15LL;
+                        bytes = (unsigned)(eb - sb);
+                        src = in_g + (size_t)(ck.x + lane) * (size_t)a.in_stride * 4 + sb;
+                        reinterpret_cast<int *>(entry + 16)[lane] = ch.y;
+                    }
+                    if (lane == 0)
+                        *reinterpret_cast<int4 *>(entry) =
+                            make_int4(it, ck.y, ck.z, k + 1 == k1 ? kTmLast : 0);
+                    const unsigned offbytes = tm_offbytes(C::DB, ck.z);
+                    unsigned total = bytes;
+    #pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_expect_tx(&full[s], total + offbytes);
+                    __syncwarp();
+                    if (lane < ck.y)
+                        bulk_g2s(raw + s * rawstage + (unsigned)(lane * a.rowcap), src, bytes, &full[s]);
+                    if (lane == 0)
+                        bulk_g2s(offsm + (n & (kTmEntries - 1)) * offstage, a.offs + (size_t)ck.w * 8,
+                                 offbytes, &full[s]);
+                    next_stage();
+                    ck = nk;
+                    ch = nch;
                 }
-                if (lane == 0)
-                    *reinterpret_cast<int4 *>(entry) =
-                        make_int4(it, ck.y, ck.z, k + 1 == k1 ? kTmLast : 0);
-                const unsigned offbytes = tm_offbytes(C::DB, ck.z);
-                unsigned total = bytes;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-                __syncwarp();
-                if (lane == 0) mbar_arrive_expect_tx(&full[s], total + offbytes);
-                __syncwarp();
-                if (lane < ck.y)
-                    bulk_g2s(raw + s * rawstage + (unsigned)(lane * a.rowcap), src, bytes, &full[s]);
-                if (lane == 0)
-                    bulk_g2s(offsm + (n & (kTmEntries - 1)) * offstage, a.offs + (size_t)ck.w * 8,
-                             offbytes, &full[s]);
-                next_stage();
-                ck = nk;
-                ch = nch;
             }
-        }
-        if (!late && claim()) {  // the end of the stream
-            if (lane == 0) {
-                *reinterpret_cast<int4 *>(meta + (n & (kTmEntries - 1)) * kTmMeta) =
-                    make_int4(-1, 0, 0, kTmStop);
-                mbar_arrive(&full[s]);
+            if (!late && claim()) {  // the end of the stream
+                if (lane == 0) {
+                    *reinterpret_cast<int4 *>(meta + (n & (kTmEntries - 1)) * kTmMeta) =
+                        make_int4(-1, 0, 0, kTmStop);
+                    mbar_arrive(&full[s]);
+                }
+            } else {
+                // let the copies already issued land before the CTA exits (bounded as well)
+                for (unsigned m = 0; m < nst; ++m)
+                    if (m < s || round > 0)
+                        mbar_wait_bounded(&full[m], (m < s ? round : round - 1u) & 1u, nullptr, 0);
             }
-        } else {
-            // let the copies already issued land before the CTA exits (bounded as well)
-            for (unsigned m = 0; m < nst; ++m)
-                if (m < s || round > 0)
-                    mbar_wait_bounded(&full[m], (m < s ? round : round - 1u) & 1u, nullptr, 0);
-        }
         }
     }
     __syncwarp();
@@ -587,9 +587,10 @@ static void tm_offsets(const StageGeom &g, const std::vector<int32_t> &S, TmStag
         }
 }
 
-// The launch's estimated clocks in this form: 17.4 a trial and channel of a block, 1550 a chunk (its channels' last pairs, the waits) and
-// an item, and the launch with its first chunks 15000; a least-squares fit to 240 launches (64-4096
-// channels, 32-3929 trials, 2295-250094 samples, spans of 0-130) with an rms error of 8%.
+// The launch's estimated clocks in this form: 17.4 a trial and channel of a block, 1550 a chunk (its
+// channels' last pairs, the waits) and an item, and the launch with its first chunks 15000; a least-squares
+// fit to 240 launches (64-4096 channels, 32-3929 trials, 2295-250094 samples, spans of 0-130) with an rms
+// error of 8%.
 static double tm_clocks(const StageGeom &g, const TmStage &t)
 {
     const double items = (double)g.ngroups * t.nblk;
